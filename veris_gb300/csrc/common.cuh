@@ -193,6 +193,42 @@ inline bool smem_configured(std::atomic<bool> (&done)[MAX_DEVICES], K kern, int 
     return true;
 }
 
+// Chained launches of a loop whose every launch reads what the one before it
+// wrote: the kernel is launched as a programmatic dependent of its
+// predecessor, so its CTAs take the slots the predecessor's last CTAs leave
+// free and the launch latency (2-3 us between two kernels of a stream) runs
+// under the predecessor's tail.  A kernel launched so
+//   * calls chain_wait() before it touches anything an earlier launch of the
+//     stream writes or reads (it returns once those launches are complete and
+//     their writes visible), and reads such data with plain loads, not
+//     through the read-only path: the array still changes while the kernel
+//     is resident;
+//   * calls chain_release() late in every CTA that does not exit before; a
+//     successor's CTAs then wait in chain_wait().
+// After a launch that does not release (any other kernel, a copy) the start
+// is the ordinary one.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;"); }
+
+template <class... P, class... A>
+inline int launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A &...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, kern, P(args)...) != cudaSuccess) {
+        cudaGetLastError();
+        return VERIS_ERR_LAUNCH;
+    }
+    return VERIS_OK;
+}
+
 }  // namespace veris
 
 #define VERIS_CHECK_GRID(g, d)                        \

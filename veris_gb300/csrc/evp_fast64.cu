@@ -145,12 +145,13 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
     auto uoc = [&](int li, int lj) { return __ldg(c.uOc + (int64_t)d.wxt(i0 + li) * lp + d.wyt(j0 + lj)); };
     auto voc = [&](int li, int lj) { return __ldg(c.vOc + (int64_t)d.wxt(i0 + li) * lp + d.wyt(j0 + lj)); };
 
+    chain_wait();
     // ---- stage u, v and the flags of the tile plus a 2-cell ring
     for (int idx = tid; idx < nS; idx += F64_THREADS) {
         const int li = idx / S::WS - 2, lj = idx % S::WS - 2;
         const int64_t o = (int64_t)d.wxt(i0 + li) * lp + d.wyt(j0 + lj);
-        sU[idx] = __ldg(io.u + o);
-        sV[idx] = __ldg(io.v + o);
+        sU[idx] = io.u[o];
+        sV[idx] = io.v[o];
         sF[idx] = __ldg(c.flags + o);
     }
     __syncthreads();
@@ -222,8 +223,8 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
             const bool mC = f0 & F_MC;
             // sigma_k = sigma_k (alpha-1)/alpha + zeta/(2 alpha) * (4 ep - 2 kp Delta | em)
             const double zh = zeta;
-            const double s1 = mC ? fma(__ldg(io.s1 + o), k.am1r, zh * fma(4.0, ep, -(k.kp2 * delta))) : 0.0;
-            const double s2 = mC ? fma(__ldg(io.s2 + o), k.am1r, zh * em) : 0.0;
+            const double s1 = mC ? fma(io.s1[o], k.am1r, zh * fma(4.0, ep, -(k.kp2 * delta))) : 0.0;
+            const double s2 = mC ? fma(io.s2[o], k.am1r, zh * em) : 0.0;
             sS11[q] = (s1 + s2) * __ldg(c.dyVh_y + gj);
             sS22[q] = (s1 - s2) * __ldg(c.dxUh_x + gi);
             const bool own = li >= 0 && lj >= 0 && i0 + li < d.NX && j0 + lj < d.NY;
@@ -279,11 +280,18 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
         const double nh = n == 4 ? k.nh4 : (n == 3 ? k.nh3 : (n == 2 ? k.nh2 : (n == 1 ? k.nh1 : 0.0)));
         const double zs = (sZeta[IB(li, lj)] + sZeta[IB(li - 1, lj)]) +
                           (sZeta[IB(li, lj - 1)] + sZeta[IB(li - 1, lj - 1)]);
-        const double s12 = fma(__ldg(io.s12 + (int64_t)gi * lp + gj), k.am1r, (nh * zs) * sE12[IZ(li, lj)]);
+        const double s12 = fma(io.s12[(int64_t)gi * lp + gj], k.am1r, (nh * zs) * sE12[IZ(li, lj)]);
         sS12[idx] = s12;
         if (li < ti && lj < S::TJ && i0 + li < d.NX && j0 + lj < d.NY) io.s12o[(int64_t)gi * io.ldo + gj] = s12;
     }
     __syncthreads();
+
+    // the next subcycle's CTAs may start: they find room as this launch's last
+    // CTAs end, and stage D covers their launch latency (released before D
+    // 191.0 us a subcycle on 1440 x 720, before C 191.4, before B 191.1, at
+    // the kernel's start 192.1, unchained 194.0; 360 x 180: 20.1, 20.5, 20.8,
+    // 21.2, 22.6)
+    chain_release();
 
     // ---- D: u, v at the tile's U and V points (veris/evp_solver.py:105-187)
     for (int base = 0; base < ti * S::TJ; base += F64_THREADS) {
@@ -357,13 +365,20 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
 #undef IZZ
 }
 
-// The units of a launch: when all full pieces fit the resident CTAs' slots
-// at once, the fewest pieces of at most TI rows; otherwise a last round of
-// about one small piece (TI/4 rows) per slot at the bottom of every strip,
-// the rest in full pieces.  (Equal full tiles left a thin last wave: 12 % of
-// the SM cycles idle on 1440 x 720 with 24-row tiles; third-height last
-// pieces took 197.2 us a launch there, quarter-height 193.0, fifth- and
-// sixth-height 193.8.)
+// The units of a launch.  When full pieces of TI rows would fit the resident
+// CTAs' slots at once, the rows are dealt out over all slots instead, down to
+// two rows a piece: a subcycle of a small grid then takes the time of a short
+// piece, although its ring is a larger part of the work (pieces of five rows
+// do a third more than they store, of two rows twice as much).  24-row pieces took 33-35 us
+// a subcycle on every grid up to 443 x 221 (8 CTAs on 90 x 40, 96 on
+// 360 x 180); over all slots 90 x 40 takes 9.5 us, 360 x 180 22.6, 443 x 221
+// 30.7, 720 x 360 59.6 (69.8 before); one piece per SM 9.6, 26.6, 34.8, 69.8;
+// one-row pieces 11.9 on 90 x 40, at least three rows 11.8 there.
+// Larger grids get a last round of about one small piece (TI/4 rows) per slot
+// at the bottom of every strip, the rest in full pieces.  (Equal full tiles
+// left a thin last wave: 12 % of the SM cycles idle on 1440 x 720 with 24-row
+// tiles; third-height last pieces took 197.2 us a launch there,
+// quarter-height 193.0, fifth- and sixth-height 193.8.)
 static F64Units f64_units(const Dims &d, int TI, int slots) {
     const int strips = (d.NY + 31) / 32;
     F64Units w;
@@ -378,6 +393,11 @@ static F64Units f64_units(const Dims &d, int TI, int slots) {
         else w.P2 = 0;
     }
     w.P1 = (w.R1 + TI - 1) / TI;
+    if ((int64_t)strips * minP <= slots) {
+        const int fit = slots / strips, two = d.NX / 2;
+        const int pieces = fit < two ? fit : two;
+        if (pieces > w.P1) w.P1 = pieces;
+    }
     w.U1 = strips * w.P1;
     return w;
 }
@@ -405,8 +425,7 @@ static int launch64(const Dims &d, int64_t lp, const HaloFill &h, const FastCons
     if (sms <= 0) return VERIS_ERR_LAUNCH;
     const F64Units w = f64_units(d, TI, per * sms);
     const int units = w.U1 + ((d.NY + S::TJ - 1) / S::TJ) * w.P2;
-    kern<<<units, F64_THREADS, sm, st>>>(d, lp, h, c, k, io, w);
-    return launch_status();
+    return launch_chained(kern, dim3(units), dim3(F64_THREADS), sm, st, d, lp, h, c, k, io, w);
 }
 
 // a taped subcycle (io.tDel set) also writes Delta, zeta and cDrag
