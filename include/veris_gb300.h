@@ -194,6 +194,23 @@ int veris_evp_solver_f64(const VerisGrid *g, const VerisParams *p, const VerisFi
                          int32_t n_subcycles, double *uIce, double *vIce, double *sigma1,
                          double *sigma2, double *sigma12, void *workspace,
                          size_t workspace_bytes, veris_stream_t s);
+/* The same loop, on any state, with the subcycle's step constants folded once
+ * per call where the state allows it (metrics varying along one axis, masks 0
+ * or 1, no curvature terms, finite inputs: checked on the device by the fold
+ * itself, no synchronisation) and the plain subcycle where it does not.  The
+ * results are those of veris_evp_solver_f64 to rounding.  The workspace size
+ * depends on the settings. */
+size_t veris_evp_auto_workspace_bytes(const VerisGrid *g, const VerisParams *p);
+int veris_evp_auto_solver_f64(const VerisGrid *g, const VerisParams *p, const VerisFieldsF64 *vs,
+                              int32_t n_subcycles, double *uIce, double *vIce, double *sigma1,
+                              double *sigma2, double *sigma12, void *workspace,
+                              size_t workspace_bytes, veris_stream_t s);
+/* The same with the residual diagnostics of veris_evp_residual_solver_f64. */
+size_t veris_evp_auto_residual_workspace_bytes(const VerisGrid *g, const VerisParams *p, int32_t n_subcycles);
+int veris_evp_auto_residual_solver_f64(const VerisGrid *g, const VerisParams *p, const VerisFieldsF64 *vs,
+                                       int32_t n_subcycles, double *uIce, double *vIce, double *sigma1,
+                                       double *sigma2, double *sigma12, double *resU, double *resSig,
+                                       void *workspace, size_t workspace_bytes, veris_stream_t s);
 int veris_evp_solver_f32(const VerisGrid *g, const VerisParams *p, const VerisFieldsF32 *vs,
                          int32_t n_subcycles, float *uIce, float *vIce, float *sigma1,
                          float *sigma2, float *sigma12, void *workspace,

@@ -141,6 +141,10 @@ SIGNATURES = {
     "veris_stressdiv_f64": ([_G, _Pa, _F, _P, _P, _P, _P, _P, _P], _I),
     "veris_evp_workspace_bytes": ([_G, ctypes.c_int32], _S),
     "veris_evp_solver_f64": ([_G, _Pa, _F, ctypes.c_int32, _P, _P, _P, _P, _P, _P, _S, _P], _I),
+    "veris_evp_auto_workspace_bytes": ([_G, _Pa], _S),
+    "veris_evp_auto_solver_f64": ([_G, _Pa, _F, ctypes.c_int32, _P, _P, _P, _P, _P, _P, _S, _P], _I),
+    "veris_evp_auto_residual_workspace_bytes": ([_G, _Pa, ctypes.c_int32], _S),
+    "veris_evp_auto_residual_solver_f64": ([_G, _Pa, _F, ctypes.c_int32] + [_P] * 8 + [_S, _P], _I),
     "veris_evp_residual_workspace_bytes": ([_G, ctypes.c_int32, ctypes.c_int32], _S),
     "veris_evp_residual_solver_f64": ([_G, _Pa, _F, ctypes.c_int32] + [_P] * 8 + [_S, _P], _I),
     "veris_evp_residual_solver_f32": ([_G, _Pa, _F, ctypes.c_int32] + [_P] * 8 + [_S, _P], _I),

@@ -160,6 +160,7 @@ struct FastIO {
     // zeta of the subcycle's viscosities and its ocean-drag coefficient,
     // which the adjoint reads instead of recomputing
     T *tDel = nullptr, *tZeta = nullptr, *tCd = nullptr;
+    T *aCo = nullptr;   // the drop-in's loop with adaptive EVP: alphaC of the subcycle (pitch ldo), when not null
 };
 
 int fast_support(const VerisParams &p);

@@ -17,14 +17,17 @@ struct Ctx {
     Dims d;
     VerisParams p;
     __device__ __forceinline__ T ld(const T *a, int i, int j) const { return __ldg(a + d.at(i, j)); }
+    // the state u, v, sigma: in a chained loop the launch before this one may still be writing it while this
+    // one becomes resident, so not through the read-only path
+    __device__ __forceinline__ T st(const T *a, int i, int j) const { return a[d.at(i, j)]; }
 };
 
 // veris/dynamics_routines.py:151-158: e11, e22 at the C point
 template <class T>
 __device__ __forceinline__ void strain_c(const Ctx<T> &c, const T *u, const T *v, int i, int j,
                                          T &e11, T &e22) {
-    const T u0 = c.ld(u, i, j), ue = c.ld(u, i + 1, j);
-    const T v0 = c.ld(v, i, j), vn = c.ld(v, i, j + 1);
+    const T u0 = c.st(u, i, j), ue = c.st(u, i + 1, j);
+    const T v0 = c.st(v, i, j), vn = c.st(v, i, j + 1);
     const T dudx = (ue - u0) * c.ld(c.f.recip_dxU, i, j);
     const T uave = (ue + u0) * T(0.5);
     const T dvdy = (vn - v0) * c.ld(c.f.recip_dyV, i, j);
@@ -37,8 +40,8 @@ __device__ __forceinline__ void strain_c(const Ctx<T> &c, const T *u, const T *v
 // veris/dynamics_routines.py:161-215: e12 at the Z point
 template <class T>
 __device__ __forceinline__ T strain_z(const Ctx<T> &c, const T *u, const T *v, int i, int j) {
-    const T u0 = c.ld(u, i, j), us = c.ld(u, i, j - 1);
-    const T v0 = c.ld(v, i, j), vw = c.ld(v, i - 1, j);
+    const T u0 = c.st(u, i, j), us = c.st(u, i, j - 1);
+    const T v0 = c.st(v, i, j), vw = c.st(v, i - 1, j);
     const T rdyU = c.ld(c.f.recip_dyU, i, j);
     const T rdxV = c.ld(c.f.recip_dxV, i, j);
     const T dudy = (u0 - us) * rdyU;
@@ -61,8 +64,8 @@ __device__ __forceinline__ T strain_z(const Ctx<T> &c, const T *u, const T *v, i
             T h2V = (mV0 - mVs) / T(3.0);
             h2U = h2U * (c.ld(mU, i - 2, j) * mUw + c.ld(mU, i + 1, j) * mU0);
             h2V = h2V * (c.ld(mV, i, j - 2) * mVs + c.ld(mV, i, j + 1) * mV0);
-            e12 = e12 + T(0.5) * (rdyU * (T(6.0) * uave - c.ld(u, i - 2, j) * mUw - c.ld(u, i + 1, j) * mU0) * h2U +
-                                  rdxV * (T(6.0) * vave - c.ld(v, i, j - 2) * mVs - c.ld(v, i, j + 1) * mV0) * h2V);
+            e12 = e12 + T(0.5) * (rdyU * (T(6.0) * uave - c.st(u, i - 2, j) * mUw - c.st(u, i + 1, j) * mU0) * h2U +
+                                  rdxV * (T(6.0) * vave - c.st(v, i, j - 2) * mVs - c.st(v, i, j + 1) * mV0) * h2V);
         }
     }
     return e12;
@@ -100,10 +103,10 @@ template <class T>
 __device__ __forceinline__ T ocean_drag_c(const Ctx<T> &c, const T *u, const T *v, int i, int j) {
     const T fc = c.ld(c.f.fCori, i, j);
     const T dc = T((double)(fc < T(0) ? c.p.waterIceDrag_south : c.p.waterIceDrag) * c.p.rhoSea);
-    const T du = (c.ld(u, i, j) - c.ld(c.f.uOcean, i, j)) * c.ld(c.f.maskInU, i, j);
-    const T due = (c.ld(u, i + 1, j) - c.ld(c.f.uOcean, i + 1, j)) * c.ld(c.f.maskInU, i + 1, j);
-    const T dv = (c.ld(v, i, j) - c.ld(c.f.vOcean, i, j)) * c.ld(c.f.maskInV, i, j);
-    const T dvn = (c.ld(v, i, j + 1) - c.ld(c.f.vOcean, i, j + 1)) * c.ld(c.f.maskInV, i, j + 1);
+    const T du = (c.st(u, i, j) - c.ld(c.f.uOcean, i, j)) * c.ld(c.f.maskInU, i, j);
+    const T due = (c.st(u, i + 1, j) - c.ld(c.f.uOcean, i + 1, j)) * c.ld(c.f.maskInU, i + 1, j);
+    const T dv = (c.st(v, i, j) - c.ld(c.f.vOcean, i, j)) * c.ld(c.f.maskInV, i, j);
+    const T dvn = (c.st(v, i, j + 1) - c.ld(c.f.vOcean, i, j + 1)) * c.ld(c.f.maskInV, i, j + 1);
     const T t = T(0.25) * (sq(du + due) + sq(dv + dvn));
     const T cmin = T(c.p.cDragMin);
     const T cd = (dc * dc * t > T(c.p.cDragMin * c.p.cDragMin)) ? dc * sqrt(t) : cmin;
@@ -115,10 +118,10 @@ template <class T>
 __device__ __forceinline__ T basal_drag_c(const Ctx<T> &c, const T *u, const T *v, int i, int j) {
     const T A = c.ld(c.f.Area, i, j);
     if (!(A > T(0.01))) return T(0.0);
-    const T um = c.ld(u, i, j) * c.ld(c.f.maskInU, i, j);
-    const T ume = c.ld(u, i + 1, j) * c.ld(c.f.maskInU, i + 1, j);
-    const T vm = c.ld(v, i, j) * c.ld(c.f.maskInV, i, j);
-    const T vmn = c.ld(v, i, j + 1) * c.ld(c.f.maskInV, i, j + 1);
+    const T um = c.st(u, i, j) * c.ld(c.f.maskInU, i, j);
+    const T ume = c.st(u, i + 1, j) * c.ld(c.f.maskInU, i + 1, j);
+    const T vm = c.st(v, i, j) * c.ld(c.f.maskInV, i, j);
+    const T vmn = c.st(v, i, j + 1) * c.ld(c.f.maskInV, i, j + 1);
     T t = T(0.25) * (um * um + ume * ume + vm * vm + vmn * vmn);
     t = T(c.p.basalDragK2) / sqrt(t + T(c.p.basalDragU0 * c.p.basalDragU0));
     const T hcrit = fabs(c.ld(c.f.R_low, i, j)) * A / T(c.p.basalDragK1);
@@ -130,7 +133,7 @@ __device__ __forceinline__ T basal_drag_c(const Ctx<T> &c, const T *u, const T *
 // veris/dynamics_routines.py:110-112: ice speed at the C point (side drag)
 template <class T>
 __device__ __forceinline__ T ice_speed_c(const Ctx<T> &c, const T *u, const T *v, int i, int j) {
-    return T(0.5) * sqrt(sq(c.ld(u, i, j) + c.ld(u, i + 1, j)) + sq(c.ld(v, i, j) + c.ld(v, i, j + 1)));
+    return T(0.5) * sqrt(sq(c.st(u, i, j) + c.st(u, i + 1, j)) + sq(c.st(v, i, j) + c.st(v, i, j + 1)));
 }
 
 // veris/dynamics_routines.py:115-138 from the speeds at C(i,j) and its west

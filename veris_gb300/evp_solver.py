@@ -18,7 +18,8 @@ def evp_solver(state, n_subcycles=None):
 
     Runs ``settings.nEVPsteps`` subcycles (or ``n_subcycles``) from the
     state's velocities and stresses in float64, one tiled kernel per
-    subcycle.  With ``settings.computeEvpResidual`` the residuals of every
+    subcycle, on constants folded once per call where the state's metrics and
+    masks allow it.  With ``settings.computeEvpResidual`` the residuals of every
     subcycle are computed as well (``evp_solver_residuals``), kept in the
     module's ``last_residuals`` and printed when its ``printEvpResidual`` is
     set, as in the reference (:227-234).
@@ -35,8 +36,8 @@ def evp_solver(state, n_subcycles=None):
     n = int(s.nEVPsteps if n_subcycles is None else n_subcycles)
     c = Call(state)
     out = c.empty(5)
-    ws, wsb = c.workspace(c.lib.veris_evp_workspace_bytes(c.refs()[0], 8))
-    check("evp_solver", c.lib.veris_evp_solver_f64(*c.refs(), n, *[t.data_ptr() for t in out], ws, wsb,
+    ws, wsb = c.workspace(c.lib.veris_evp_auto_workspace_bytes(*c.refs()[:2]))
+    check("evp_solver", c.lib.veris_evp_auto_solver_f64(*c.refs(), n, *[t.data_ptr() for t in out], ws, wsb,
                                                     c.stream))
     return tuple(out)
 
@@ -60,9 +61,12 @@ def evp_solver_residuals(state, n_subcycles=None, precision="f64"):
     c = Call(state, dtype=dt)
     out = c.empty(5)
     res = torch.zeros((2, max(n, 1)), dtype=torch.float64, device=c.device)
-    ws, wsb = c.workspace(c.lib.veris_evp_residual_workspace_bytes(c.refs()[0], 4 if dt == torch.float32 else 8,
-                                                                   n))
-    fn = c.lib.veris_evp_residual_solver_f32 if dt == torch.float32 else c.lib.veris_evp_residual_solver_f64
+    if dt == torch.float32:
+        size, fn = c.lib.veris_evp_residual_workspace_bytes(c.refs()[0], 4, n), c.lib.veris_evp_residual_solver_f32
+    else:
+        size = c.lib.veris_evp_auto_residual_workspace_bytes(*c.refs()[:2], n)
+        fn = c.lib.veris_evp_auto_residual_solver_f64
+    ws, wsb = c.workspace(size)
     check("evp_solver_residuals", fn(*c.refs(), n, *[t.data_ptr() for t in out], res[0].data_ptr(),
                                      res[1].data_ptr(), ws, wsb, c.stream))
     return tuple(out) + (res[0, :n], res[1, :n])
