@@ -688,6 +688,9 @@ int veris_convert_f32_to_f64(const float *src, double *dst, int64_t n, veris_str
  * (sqrt of -0 in the warp form: +0 when the warp takes the series).
  */
 int veris_f64_math_check(const double *a, const double *b, int64_t n, double *out, veris_stream_t s);
+/* The float64 kernels' table-driven exp(x), log(x) and atan(x), planar in out
+ * (3 n values), for checking them against correctly rounded results. */
+int veris_f64_functions_check(const double *x, int64_t n, double *out, veris_stream_t s);
 
 #ifdef __cplusplus
 }

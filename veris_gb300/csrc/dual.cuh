@@ -10,6 +10,8 @@
 
 #include <cuda_runtime.h>
 
+#include "f64math.cuh"
+
 namespace veris {
 
 template <int N>
@@ -141,18 +143,33 @@ __device__ inline Dual<N> vfabs(const Dual<N> &a) {
 
 // the same names for plain float64, so templated code calls one spelling
 __device__ inline double vsqrt(double x) { return ::sqrt(x); }
-__device__ inline double vrsqrt(double x) { return ::rsqrt(x); }
-__device__ inline double vexp(double x) { return ::exp(x); }
+__device__ inline double vrsqrt(double x) { return rsqrt_lane(x); }
+__device__ inline double vexp(double x) { return exp_table(x); }
 __device__ inline double vexp10(double x) { return ::exp10(x); }
 __device__ inline double vexp2(double x) { return ::exp2(x); }
 __device__ inline double vlog(double x) { return ::log(x); }
+__device__ inline double vdiv(double a, double b) { return div_lane(a, b); }
+template <int N>
+__device__ inline Dual<N> vdiv(double a, const Dual<N> &b) { return a / b; }
 __device__ inline double vfabs(double x) { return ::fabs(x); }
 __device__ inline float vfabs(float x) { return ::fabsf(x); }
 
+// comparisons of values (false on NaN, as the operators'), on the integer pipe
+template <class S>
+__device__ inline bool vpos(const S &x) { return is_pos(val(x)); }   // x > 0
+template <class S>
+__device__ inline bool vzero(const S &x) { return is_zero(val(x)); }
+template <class S>
+__device__ inline bool vge(const S &a, const S &b) { return ge64(val(a), val(b)); }
+template <class S>
+__device__ inline bool vle0(const S &x) { return !is_pos(val(x)) && !is_nan64(val(x)); }   // x <= 0
+template <class S>
+__device__ inline bool vgt(const S &a, const S &b) { return gt64(val(a), val(b)); }
+
 // select-type min/max: the chosen operand's derivatives (first one on ties)
 template <class S>
-__device__ inline S smax(const S &a, const S &b) { return a > b ? a : b; }
+__device__ inline S smax(const S &a, const S &b) { return vgt(a, b) ? a : b; }
 template <class S>
-__device__ inline S smin(const S &a, const S &b) { return a < b ? a : b; }
+__device__ inline S smin(const S &a, const S &b) { return vgt(b, a) ? a : b; }
 
 }  // namespace veris

@@ -60,10 +60,6 @@ static size_t auto_layout(const Dims &d, const VerisParams &p, char *base, AutoS
     return off;
 }
 
-__device__ __forceinline__ bool finite64(double x) {
-    return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
-}
-
 // Folds the step's constants and checks the state.  Non-finite inputs take
 // the plain tile too: it multiplies by the masks, so that a NaN on land
 // spreads as in the reference, where the folded form selects.

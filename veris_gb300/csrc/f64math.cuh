@@ -14,6 +14,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "f64tables.cuh"
+
 namespace veris {
 
 __device__ __forceinline__ double rcp_seed(double b) {
@@ -125,5 +127,110 @@ __device__ __forceinline__ double sqrt_lane(double x) {
     return seed_range(x) ? sqrt_series(x) : sqrt(x);
 }
 __device__ __forceinline__ double rsqrt_lane(double x) { return seed_range(x) ? rsqrt_series(x) : 1.0 / sqrt(x); }
+
+// ------------------------------------------------ tests on the integer pipe
+// Comparisons of float64 values cost a slot of the float64 pipe each; on the
+// bits they run on the integer pipe.  As the float comparisons, they are
+// false where an operand is NaN.
+__device__ __forceinline__ bool is_nan64(double x) { return (bits_of(x) << 1) > 0xffe0000000000000ULL; }
+__device__ __forceinline__ bool finite64(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+// the bits as a signed integer in the order of the values (-0 just below +0)
+__device__ __forceinline__ long long order64(double x) {
+    const long long b = (long long)bits_of(x);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+__device__ __forceinline__ bool is_pos(double x) {   // x > 0
+    const long long b = (long long)bits_of(x);
+    return b > 0 && b <= 0x7ff0000000000000LL;
+}
+__device__ __forceinline__ bool is_neg(double x) {   // x < 0
+    const unsigned long long b = bits_of(x);
+    return b > 0x8000000000000000ULL && b <= 0xfff0000000000000ULL;
+}
+__device__ __forceinline__ bool gt64(double a, double b) {   // a > b
+    return order64(a) > order64(b) && !is_nan64(a) && !is_nan64(b) && !(is_zero(a) && is_zero(b));
+}
+
+__device__ __forceinline__ bool ge64(double a, double b) {   // a >= b
+    return !gt64(b, a) && !is_nan64(a) && !is_nan64(b);
+}
+
+// ------------------------------- float32 <-> float64 on the integer pipe
+// a normal float, exactly (0 gives 2^-127 with its sign, for correction terms)
+__device__ __forceinline__ double widen(float x) {
+    const unsigned b = __float_as_uint(x);
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+// truncated to float; magnitudes below 2^-126 become about 2^-126, those
+// above the float range infinite or NaN: for approximations and tails
+__device__ __forceinline__ float narrow(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned e = min(max(hi & 0x7fffffffu, 0x38100000u), 0x47f00000u) - 0x38000000u;
+    return __uint_as_float((hi & 0x80000000u) | (e << 3) | (lo >> 29));
+}
+
+// ------------------------------------------- exponential, logarithm, arctangent
+// Table-driven (P. T. P. Tang, ACM Trans. Math. Softw. 15 (1989) 144 and 16
+// (1990) 378): the tables of f64tables.cuh leave a remainder so small that
+// the last terms of its series, below 2^-30 of the result, are evaluated in
+// float32, and the float64 pipe sees eight, seven and eleven operations.
+
+// e^x for |x| <= 700: x = (512 n + k) ln2/512 + r, |r| <= ln2/1024; e^x = 2^n
+// 2^(k/512) (1 + r + r^2 (1/2 + r/6 + r^2/24))
+__device__ __forceinline__ double exp_core(double x) {
+    const double magic = 6755399441055744.0;   // 1.5 * 2^52: the sum's low word is the rounded integer
+    const double s = fma(x, 0x1.71547652b82fep+9, magic);
+    const int n = __double2loint(s);
+    const double k = s - magic;
+    const double r = fma(k, -0x1.473de6af278edp-43, fma(k, -0x1.62e42fef00000p-10, x));
+    const float f = narrow(r);
+    const double q = 0.5 + widen(f * fmaf(f, 1.f / 24.f, 1.f / 6.f));
+    const double p = fma(r * r, q, r);
+    const double T = __ldg(EXP2_512 + (n & 511));
+    const double e = fma(T, p, T);
+    return __hiloint2double(__double2hiint(e) + ((n >> 9) << 20), __double2loint(e));
+}
+// any x: beyond the core's range the square of e^(x/2), up to overflow and to the subnormals
+static __device__ __noinline__ double exp_far(double x) {
+    if (is_nan64(x)) return x;
+    if (gt64(x, 1400.0)) return __hiloint2double(0x7ff00000, 0);
+    if (gt64(-1400.0, x)) return 0.0;
+    const double e = exp_core(0.5 * x);
+    return e * e;
+}
+__device__ __forceinline__ double exp_table(double x) {
+    return (unsigned)(__double2hiint(x) & 0x7fffffff) < 0x4085e000u ? exp_core(x) : exp_far(x);
+}
+
+// log(x) for x = 2^e m in [1, 2^64): with r = m c - 1, c ~ 1/m from the table,
+// log x = e ln2 - log c + r + r^2 (-1/2 + r (1/3 + r (-1/4 + r/5))).  Other x: log().
+__device__ __forceinline__ double log_table(double x) {
+    const int hi = __double2hiint(x);
+    if ((unsigned)(hi - 0x3ff00000) >= (64u << 20)) return ::log(x);
+    const double m = __hiloint2double((hi & 0x000fffff) | 0x3ff00000, __double2loint(x));
+    const double2 c = __ldg(LOG_256 + ((hi >> 12) & 255));
+    const double r = fma(m, c.x, -1.0);
+    const float f = narrow(r);
+    const double t = widen(f * fmaf(f, fmaf(f, -1.f / 6.f, 0.2f), -0.25f));
+    const double p = fma(r * r, fma(r, 1.0 / 3.0 + t, -0.5), r);
+    const int e = (hi - 0x3ff00000) >> 20;
+    double L = c.y;
+    if (e != 0) L = fma(widen((float)e), 0.6931471805599453094, L);
+    return L + p;
+}
+
+// atan(x) for x in [1, 3.6]: with c the nearest 1 + k/64 and d = (x - c)/(1 + x c),
+// atan x = atan c + d + d^3 (-1/3 + d^2 (1/5 - d^2/7)).  Other x: atan().
+__device__ __forceinline__ double atan_table(double x) {
+    const int hi = __double2hiint(x);
+    if ((unsigned)(hi - 0x3ff00000) > (unsigned)(0x400ccccc - 0x3ff00000)) return ::atan(x);
+    const int k = (int)fmaf(narrow(x), 64.f, -63.5f);   // 64 (x - 1), rounded
+    const double c = widen(fmaf((float)k, 0.015625f, 1.f));
+    const double d = div_series(x - c, fma(x, c, 1.0));
+    const double d2 = d * d;
+    const float f = narrow(d2);
+    const double q = widen(f * fmaf(f, -1.f / 7.f, 0.2f)) - 1.0 / 3.0;
+    return __ldg(ATAN_64 + k) + fma(d * d2, q, d);
+}
 
 }  // namespace veris

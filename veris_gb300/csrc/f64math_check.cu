@@ -2,7 +2,8 @@
 // f64math.cuh (the float64 EVP subcycle, its adjoint, the free drift and the
 // bulk formula use them in place of IEEE division and square root): each
 // form evaluated elementwise, so that a caller can measure them against
-// correctly rounded results and IEEE special values.
+// correctly rounded results and IEEE special values; and of its table-driven
+// exponential, logarithm and arctangent (Growth, the bulk formula).
 #include "common.cuh"
 #include "f64math.cuh"
 
@@ -32,6 +33,15 @@ __global__ void __launch_bounds__(CHECK_THREADS) f64math_check_kernel(const doub
     out[7 * n + i] = rsqrt_lane(y);
 }
 
+// out (planar, n each): exp_table(x), log_table(x), atan_table(x)
+__global__ void __launch_bounds__(CHECK_THREADS) f64functions_check_kernel(const double *x, int64_t n, double *out) {
+    const int64_t i = (int64_t)blockIdx.x * CHECK_THREADS + threadIdx.x;
+    if (i >= n) return;
+    out[i] = exp_table(x[i]);
+    out[n + i] = log_table(x[i]);
+    out[2 * n + i] = atan_table(x[i]);
+}
+
 }  // namespace
 
 }  // namespace veris
@@ -43,5 +53,15 @@ extern "C" int veris_f64_math_check(const double *a, const double *b, int64_t n,
     const int64_t blocks = (n + veris::CHECK_THREADS - 1) / veris::CHECK_THREADS;
     VERIS_REQUIRE(blocks <= 0x7fffffff, VERIS_ERR_ARG);
     veris::f64math_check_kernel<<<(unsigned)blocks, veris::CHECK_THREADS, 0, (cudaStream_t)s>>>(a, b, n, out);
+    return veris::launch_status();
+}
+
+extern "C" int veris_f64_functions_check(const double *x, int64_t n, double *out, veris_stream_t s) {
+    VERIS_REQUIRE(n >= 0, VERIS_ERR_ARG);
+    if (n == 0) return VERIS_OK;
+    VERIS_REQUIRE(x && out, VERIS_ERR_ARG);
+    const int64_t blocks = (n + veris::CHECK_THREADS - 1) / veris::CHECK_THREADS;
+    VERIS_REQUIRE(blocks <= 0x7fffffff, VERIS_ERR_ARG);
+    veris::f64functions_check_kernel<<<(unsigned)blocks, veris::CHECK_THREADS, 0, (cudaStream_t)s>>>(x, n, out);
     return veris::launch_status();
 }
