@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(256) bulkf_kernel(BulkArgs<T> a) {
 //   psi_h = 2 ln((1 + x^2)/2), x = (1 - 16 huol)^(1/4);
 //   Dm, Dh = 1 + g (aln - psi) = c0 - g psi
 // 1444 x 724 points, half of them unstable: 1.50 ms with CUDA's log, atan and
-// exp (170 operations per unstable iteration); here 0.61 ms.
+// exp (170 operations per unstable iteration); here 0.67 ms.
 __global__ void __launch_bounds__(256) bulkf64_kernel(BulkArgs<double> a, double c0) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < a.n;
          k += (int64_t)gridDim.x * blockDim.x) {

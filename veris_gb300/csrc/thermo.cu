@@ -2,10 +2,8 @@
 // (veris/solve4temp.py:5-174) and ice growth with the ocean budgets
 // (veris/growth.py:8-397).  Both are pointwise; one thread per padded point.
 #include <cmath>
-#include <type_traits>
 
 #include "stencil.cuh"
-#include "dual.cuh"
 #include "ffmath.cuh"
 
 namespace veris {
@@ -99,11 +97,14 @@ struct GrowthK {
     // open water: conductivity and penetrating fractions of the thinnest ice, the ocean's melting rate per K,
     // recip_hIceMean
     double k0b, penb[5], meltb, rhb;
+    // the adjoint's: qsub / qnum and aa1 ln10 of the saturation humidity, 1 / (iceConduct snowConduct)
+    double qratio, aln10, rkk;
     double t2;            // Stanton number times friction velocity, density and heat capacity of the ocean
     double pFac[5];       // thickness of category l of five over the mean
     // solve4temp's saturation terms: qnum = bb1 cc0 and qsub = (1 - bb1) cc0, each as the sum of two
     // floats, and cc1
     float k0b_h, k0b_l;
+    float odd_h[5], odd_l[5];   // 1 / (2l+1)
     float qn_h, qn_l, qs_h, qs_l, cc1;
     float d3s_h, d3s_l, d3i_h, d3i_l;   // emissivity times Stefan-Boltzmann over snow and ice
     float Tmin_f, Tmelt_f;
@@ -133,9 +134,13 @@ static GrowthK growth_k(const VerisParams &p) {
     k.k0b = p.iceConduct * p.snowConduct / (p.snowConduct * (0.05 * k.pFac[0]));
     split(k.k0b, k.k0b_h, k.k0b_l);
     for (int l = 0; l < 5; ++l) k.penb[l] = p.shortwave * std::exp(-1.5 * (0.05 * k.pFac[l]));
+    for (int l = 0; l < 5; ++l) split(1.0 / (2 * l + 1), k.odd_h[l], k.odd_l[l]);
     k.t2 = p.stantonNr * p.uStarBase * p.rhoSea * p.cpWater;
     k.meltb = -k.t2 * (1 + (p.McPheeTaperFac - 1) / (1 + std::exp(-0.4 * (7 / 0.4)))) * k.qi;
     k.rhb = 1 / std::sqrt(p.hIce_reg);
+    k.qratio = qsub / qnum;
+    k.aln10 = 2663.5 * std::log(10.0);
+    k.rkk = 1 / (p.iceConduct * p.snowConduct);
     split(qnum, k.qn_h, k.qn_l);
     split(qsub, k.qs_h, k.qs_l);
     k.cc1 = (float)p.s4t_cc1;
@@ -209,277 +214,203 @@ __device__ __forceinline__ Ff saturation_ff(float t, Ff qnum, Ff qsub, float cc1
 // 1.66 ms; with the saturation term alone in double-float 0.65 ms; with the
 // whole residual in it and the short form of open water (two thirds of a
 // global grid's points) 0.45 ms.
+struct S4TCell {
+    double lwc, Ta, d1ug, d1iug, slope, aI, aS, iceSW;
+    double k0, e, e2;           // conductivity of the thinnest of five; exp(-1.5 hI[l]) of the next category, its step
+    Ff k0f, d1u, d1i, Taf, aqh, TF;
+    float Tin;
+};
+
+// what the adjoint reads of a category at its root: saturation humidity,
+// conductivity, d absSW / d thickness (of the snow, or of the ice where there is none)
+struct S4TRoot {
+    double qs, k, dSW;
+    bool up;
+};
+
+// what the categories share
 template <int NC, bool BARE>
-__device__ __forceinline__ bool solve4temp_f64(const VerisParams &p, const GrowthK &gk, const S4TIn &x, double Tin,
-                                               const double *hI, const double *hS, double *oT, double *oFio,
-                                               double *oFia, double *oPen) {
-    const double Tmelt = p.celsius2K;
-    const double lwc = dmax(p.minLWdown, x.LWdown);
-    const double Ta = dmax(gk.TaMin, x.ATemp);
+__device__ __forceinline__ S4TCell solve4temp_cell(const VerisParams &p, const GrowthK &gk, const S4TIn &x,
+                                                   double Tin, double hI0, double hS0) {
+    S4TCell c;
+    c.lwc = dmax(p.minLWdown, x.LWdown);
+    c.Ta = dmax(gk.TaMin, x.ATemp);
     const double ug = dmax(p.wSpeedMin, x.wSpeed);
-    const double d1ug = p.s4t_d1 * ug, d1iug = p.s4t_d1i * ug;
+    c.d1ug = p.s4t_d1 * ug;
+    c.d1iug = p.s4t_d1i * ug;
     const bool wet = !gt64(gk.Twet, Tin) && !is_nan64(Tin), south = is_neg(x.fCori);
-    const double aI = south ? (wet ? p.wetIceAlb_south : p.dryIceAlb_south) : (wet ? p.wetIceAlb : p.dryIceAlb);
-    const double aS = south ? (wet ? p.wetSnowAlb_south : p.drySnowAlb_south) : (wet ? p.wetSnowAlb : p.drySnowAlb);
-    const double slope = gk.rhCut * (aS - aI);
-    const double iceSW = (1 - aI) * x.SWdown;   // absorbed and transmitted by snow-free ice
+    c.aI = south ? (wet ? p.wetIceAlb_south : p.dryIceAlb_south) : (wet ? p.wetIceAlb : p.dryIceAlb);
+    c.aS = south ? (wet ? p.wetSnowAlb_south : p.drySnowAlb_south) : (wet ? p.wetSnowAlb : p.drySnowAlb);
+    c.slope = gk.rhCut * (c.aS - c.aI);
+    c.iceSW = (1 - c.aI) * x.SWdown;   // absorbed and transmitted by snow-free ice
     // the five categories scale ice and snow thickness alike (veris/growth.py:62-71): hI[l] = (2l+1) hI[0]
     // and hS[l] = (2l+1) hS[0], so one conductivity and one exponential serve them all
-    Ff k0{0.f, 0.f};
-    double k0d = 0.0, e = 0.0, e2 = 0.0;
-    bool finite = true;
+    c.k0 = c.e = c.e2 = 0.0;
     if (BARE) {
-        k0d = gk.k0b;
-        k0 = Ff{gk.k0b_h, gk.k0b_l};
+        c.k0 = gk.k0b;
+        c.k0f = Ff{gk.k0b_h, gk.k0b_l};
     } else if (NC == 5) {
-        if (is_pos(hI[0])) k0d = div_lane(p.iceConduct * p.snowConduct, fma(p.snowConduct, hI[0], p.iceConduct * hS[0]));
-        k0 = ff_of(k0d);
-        if (!is_pos(hS[0])) {   // exp(-1.5 hI[l]) = exp(-1.5 hI[0])^(2l+1)
-            e = exp_table(-1.5 * hI[0]);
-            e2 = e * e;
+        if (is_pos(hI0)) c.k0 = div_lane(p.iceConduct * p.snowConduct, fma(p.snowConduct, hI0, p.iceConduct * hS0));
+        c.k0f = ff_of(c.k0);
+        if (!is_pos(hS0)) {   // exp(-1.5 hI[l]) = exp(-1.5 hI[0])^(2l+1)
+            c.e = exp_table(-1.5 * hI0);
+            c.e2 = c.e * c.e;
         }
     }
-    const Ff d1u = ff_of(d1ug), d1i = ff_of(d1iug), Taf = ff_of(Ta), aqh = ff_of(x.aqh), TF = ff_of(x.TempFrz);
-    const Ff qnum{gk.qn_h, gk.qn_l}, qsub{gk.qs_h, gk.qs_l};
-    const float Tinf = narrow(Tin);
-#pragma unroll
-    for (int l = 0; l < NC; ++l) {
-        const bool ice = BARE || is_pos(hI[NC == 5 ? 0 : l]), snow = !BARE && is_pos(hS[l]);
-        if (!ice) {
-            oT[l] = Tin;
-            oFio[l] = oFia[l] = oPen[l] = 0.0;
-            continue;
-        }
-        const double emiss = snow ? p.snowEmiss : p.iceEmiss;
-        double absSW = iceSW;
-        if (!BARE) oPen[l] = 0.0;
-        if (snow) {
-            double alb = fma(hS[l], slope, aI);
-            if (gt64(hS[l], p.hCut)) alb = aS;
-            absSW = (1 - alb) * x.SWdown;
-        } else {
-            if (NC != 5) e = exp_table(-1.5 * hI[l]);
-            const double pen = BARE ? gk.penb[l] : p.shortwave * e;
-            if (NC == 5) e *= e2;
-            if (!BARE) oPen[l] = -iceSW * pen;
-            absSW = fma(-iceSW, pen, iceSW);
-        }
-        Ff k;
-        double kd = 0.0;
-        if (NC == 5) {
-            constexpr double inv_odd[5] = {1.0, 1.0 / 3.0, 1.0 / 5.0, 1.0 / 7.0, 1.0 / 9.0};
-            const double q = inv_odd[l];   // a constant once unrolled
-            k = ff_mul(k0, Ff{(float)q, (float)(q - (double)(float)q)});
-        } else {
-            kd = div_lane(p.iceConduct * p.snowConduct, fma(p.snowConduct, hI[l], p.iceConduct * hS[l]));
-            k = ff_of(kd);
-        }
-        const double lwabs = fma(-emiss, lwc, -absSW);
-        const Ff lw = ff_of(lwabs), d3 = snow ? Ff{gk.d3s_h, gk.d3s_l} : Ff{gk.d3i_h, gk.d3i_l};
-        float t = Tinf;
-        for (int it = 0; it < 4; ++it) {
-            const float rt = __frcp_rn(t), t2 = t * t;
-            const float c3 = exp2f(8847.95548f * rt);
-            const float D = c3 * 100000.f - gk.qs_h, rD = __frcp_rn(D);
-            const float qs = gk.qn_h * rD;
-            const float dqs = (gk.cc1 * c3 * rD) * rD * (rt * rt);
-            const float R = k.h * (TF.h - t) - (lw.h + t2 * t2 * d3.h + d1u.h * (t - Taf.h) + d1i.h * (qs - aqh.h));
-            const float dF = 4.f * d3.h * t2 * t + d1u.h + d1i.h * dqs;
-            t = fminf(fmaxf(t + R * __frcp_rn(k.h + dF), gk.Tmin_f), gk.Tmelt_f);
-        }
-        float dqs;
-        const Ff qs = saturation_ff(t, qnum, qsub, gk.cc1, dqs);
-        const float t2 = __fmul_rn(t, t);
-        const Ff tt = ff_fast_sum(t2, fmaf(t, t, -t2));
-        Ff Fc = ff_mul(k, ff_add(TF, -t));
-        Ff Fia = ff_add(ff_mul(ff_mul(tt, tt), d3), lw);
-        Fia = ff_add(Fia, ff_mul(d1u, ff_add(ff_neg(Taf), t)));
-        Fia = ff_add(Fia, ff_mul(d1i, ff_add(qs, ff_neg(aqh))));
-        const float res = (Fc.h - Fia.h) + (Fc.l - Fia.l);
-        const float dF = 4.f * d3.h * t2 * t + d1u.h + d1i.h * dqs;
-        const float step = res * __frcp_rn(k.h + dF);
-        const float tn = fminf(fmaxf(t + step, gk.Tmin_f), gk.Tmelt_f);
-        const double td = widen(t);
-        double T;
-        if (fabsf(tn - t) <= 4e-7f * t && fabsf(step) < 1e30f) {
-            T = td + widen(step);
-            float d = step;
-            if (gt64(T, Tmelt)) {
-                T = Tmelt;
-                d = narrow(Tmelt - td);
-            }
-            if (gt64(gk.Tmin, T)) {
-                T = gk.Tmin;
-                d = narrow(gk.Tmin - td);
-            }
-            if (!BARE) {
-                const float kd1 = __fmul_rn(k.h, d);
-                Fc = ff_add(Fc, Ff{-kd1, -(fmaf(k.h, d, -kd1) + k.l * d)});
-                Fia = ff_add(Fia, fmaf(6.f * d3.h * t2, d, dF) * d);
-                const bool up = Fc.h > 0.f;
-                const double F = ff_value(up ? Fc : Fia);
-                oFio[l] = up ? F : 0.0;
-                oFia[l] = up ? 0.0 : F;
-            }
-        } else {
-            // veris/solve4temp.py:108-160: six iterations and the fluxes at their end
-            const double qnumd = 0.622 * p.s4t_cc0, qsubd = (1.0 - 0.622) * p.s4t_cc0, d3d = emiss * p.stefBoltz;
-            if (NC == 5) kd = k0d * (1.0 / (2 * l + 1));
-            double Fcd = 0.0, Fiad = 0.0;
-            T = td;
-            for (int it = 0; it < 7; ++it) {
-                const double rt = 1.0 / T, c3 = ::exp2(2663.5 * 3.32192809488736234787 * rt);
-                const double s2 = T * T, D = c3 * 100000.0 - qsubd, q = qnumd / D;
-                Fcd = kd * (x.TempFrz - T);
-                Fiad = lwabs + s2 * s2 * d3d + d1ug * (T - Ta) + d1iug * (q - x.aqh);
-                if (it == 6) break;
-                const double Q = p.s4t_cc1 * c3 * (rt * rt) / (D * D);
-                T = T + (Fcd - Fiad) / (kd + 4 * d3d * (s2 * T) + d1ug + d1iug * Q);
-                T = dmax(dmin(T, Tmelt), gk.Tmin);
-            }
-            const bool up = is_pos(Fcd);
-            if (!BARE) {
-                oFio[l] = up ? Fcd : 0.0;
-                oFia[l] = up ? 0.0 : Fiad;
-            } else if (!finite64(up ? Fcd : Fiad)) {
-                finite = false;
-            }
-        }
-        oT[l] = T;
-    }
-    return finite;
+    c.d1u = ff_of(c.d1ug);
+    c.d1i = ff_of(c.d1iug);
+    c.Taf = ff_of(c.Ta);
+    c.aqh = ff_of(x.aqh);
+    c.TF = ff_of(x.TempFrz);
+    c.Tin = narrow(Tin);
+    return c;
 }
 
-// The same for dual numbers, when the adjoint needs the derivatives with
-// respect to the ice state (branches follow the values).
-template <int NC, class S>
-__device__ void solve4temp_dual(const VerisParams &p, const GrowthK &gk, const S4TIn &x, const S &Tin, const S *hI, const S *hS,
-                                S *oT, S *oFio, S *oFia, S *oPen) {
-    const double aa1 = 2663.5, bb1 = 0.622, Pa = 100000.0;
-    const double one_m_bb1 = 1.0 - bb1;
-    const double cc0 = p.s4t_cc0, cc1 = p.s4t_cc1, cc2 = p.s4t_cc2, d1 = p.s4t_d1, d1i = p.s4t_d1i;
-    const double Tmelt = p.celsius2K, Tmin = p.celsius2K + p.minTIce;
-    const double SurfMeltTemp = Tmelt + p.wetAlbTemp;
-    const double lwc = dmax(p.minLWdown, x.LWdown);
-    const double Ta = dmax(p.celsius2K + p.minTAir, x.ATemp);
-    const double ug = dmax(p.wSpeedMin, x.wSpeed);
-    const double d1ug = d1 * ug, d1iug = d1i * ug;
-    S k[NC], lwabs[NC];
-    double d3[NC];
-    bool ice[NC];
-    // penetrating shortwave factor exp(-1.5 hI): the NC = 5 categories of one
-    // cell have hI[l] = (2l+1) hI[0], so one exp and its odd powers serve all
-    S e1[NC];
-    if constexpr (NC == 5) {
-        const S E = vexp(-1.5 * hI[0]), E2 = E * E;
-        e1[0] = E;
-#pragma unroll
-        for (int l = 1; l < NC; ++l) e1[l] = e1[l - 1] * E2;
+// category l, of ice thickness hI > 0 and snow thickness hS; T, Fio, Fia, pen
+// as solve4temp returns them.  False where (BARE) a flux is not finite.
+template <int NC, bool BARE>
+__device__ __forceinline__ bool solve4temp_category(const VerisParams &p, const GrowthK &gk, const S4TIn &x,
+                                                    S4TCell &c, int l, double hI, double hS, double &T, double &Fio,
+                                                    double &Fia, double &oPen, S4TRoot *root = nullptr) {
+    const bool snow = !BARE && is_pos(hS);
+    const double emiss = snow ? p.snowEmiss : p.iceEmiss;
+    double absSW = c.iceSW;
+    oPen = 0.0;
+    if (snow) {
+        double alb = fma(hS, c.slope, c.aI);
+        const bool deep = gt64(hS, p.hCut);
+        if (deep) alb = c.aS;
+        absSW = (1 - alb) * x.SWdown;
+        if (root) root->dSW = deep ? 0.0 : -c.slope * x.SWdown;
     } else {
-#pragma unroll
-        for (int l = 0; l < NC; ++l) e1[l] = vexp(-1.5 * hI[l]);
+        if (NC != 5) c.e = exp_table(-1.5 * hI);
+        const double pen = BARE ? gk.penb[l] : p.shortwave * c.e;
+        if (!BARE && NC == 5) c.e *= c.e2;
+        if (!BARE) oPen = -c.iceSW * pen;
+        absSW = fma(-c.iceSW, pen, c.iceSW);
+        if (root) root->dSW = 1.5 * c.iceSW * pen;
     }
-    const double rhCut = gk.rhCut;
-    // the categories scale ice and snow thickness alike (veris/growth.py:62-71):
-    // with NC = 5, hI[l] = (2l+1) hI[0] and hS[l] = (2l+1) hS[0], so the
-    // effective conductivity is k[0] / (2l+1): one division for the five
-    S k0 = S(0.0);
-    if constexpr (NC == 5)
-        k0 = hI[0] > 0 ? p.iceConduct * p.snowConduct / (p.snowConduct * hI[0] + p.iceConduct * hS[0]) : S(0.0);
-#pragma unroll
-    for (int l = 0; l < NC; ++l) {
-        ice[l] = hI[l] > 0;
-        const bool snow = hS[l] > 0;
-        const double emiss = snow ? p.snowEmiss : p.iceEmiss;
-        d3[l] = emiss * p.stefBoltz;
-        const double lw = emiss * lwc;
-        double aI = ice[l] ? p.dryIceAlb : 0.0;
-        double aS = ice[l] ? p.drySnowAlb : 0.0;
-        if (ice[l] && Tin >= SurfMeltTemp) { aI = p.wetIceAlb; aS = p.wetSnowAlb; }
-        const bool south = ice[l] && x.fCori < 0;
-        if (south) { aI = p.dryIceAlb_south; aS = p.drySnowAlb_south; }
-        if (south && Tin >= SurfMeltTemp) { aI = p.wetIceAlb_south; aS = p.wetSnowAlb_south; }
-        S alb = ice[l] ? aI + hS[l] * rhCut * (aS - aI) : S(0.0);
-        if (hS[l] > p.hCut) alb = S(aS);
-        if (hS[l] == 0) alb = S(aI);
-        S pen = ice[l] ? p.shortwave * e1[l] : S(0.0);
-        if (snow) pen = S(0.0);
-        oPen[l] = ice[l] ? -(1 - alb) * pen * x.SWdown : S(0.0);
-        const S absSW = ice[l] ? (1 - alb) * (1 - pen) * x.SWdown : S(0.0);
-        if constexpr (NC == 5) {
-            constexpr double inv_odd[5] = {1.0, 1.0 / 3.0, 1.0 / 5.0, 1.0 / 7.0, 1.0 / 9.0};
-            k[l] = ice[l] ? k0 * inv_odd[l] : S(0.0);
-        } else {
-            k[l] = ice[l] ? p.iceConduct * p.snowConduct / (p.snowConduct * hI[l] + p.iceConduct * hS[l]) : S(0.0);
-        }
-        lwabs[l] = -lw - absSW;
+    Ff k;
+    double kd = 0.0;
+    if (NC == 5) {
+        k = ff_mul(c.k0f, Ff{gk.odd_h[l], gk.odd_l[l]});
+    } else {
+        kd = div_lane(p.iceConduct * p.snowConduct, fma(p.snowConduct, hI, p.iceConduct * hS));
+        k = ff_of(kd);
     }
-    // Derivatives (dual numbers): implicit differentiation at the root.
-    // The values come from the float64 solve itself (so every later
-    // branch is taken as in the forward); at its root T* of
-    // R(T) = Fc(T) - Fia(T), dT* = -R_theta / R_T with R_theta the
-    // residual's derivative at fixed T (through the conductivity and
-    // the absorbed radiation) and R_T = -(k + dFia/dT), the Newton
-    // iteration's own denominator; a root held by the melt or the
-    // minimum-temperature clamp has dT* = 0.  The converged Newton
-    // iterates have this derivative (the Newton map's derivative in T
-    // vanishes at the root), without iterating the dual numbers.
-    double hIv[NC], hSv[NC], Tv[NC], Fiov[NC], Fiav[NC], Penv[NC];
-#pragma unroll
-    for (int l = 0; l < NC; ++l) {
-        hIv[l] = val(hI[l]);
-        hSv[l] = val(hS[l]);
+    const double lwabs = fma(-emiss, c.lwc, -absSW);
+    const Ff lw = ff_of(lwabs), d3 = snow ? Ff{gk.d3s_h, gk.d3s_l} : Ff{gk.d3i_h, gk.d3i_l};
+    const Ff qnum{gk.qn_h, gk.qn_l}, qsub{gk.qs_h, gk.qs_l};
+    float t = c.Tin;
+#pragma unroll 1
+    for (int it = 0; it < 4; ++it) {
+        const float rt = __frcp_rn(t), t2 = t * t;
+        const float c3 = exp2f(8847.95548f * rt);
+        const float D = c3 * 100000.f - gk.qs_h, rD = __frcp_rn(D);
+        const float qs = gk.qn_h * rD;
+        const float dqs = (gk.cc1 * c3 * rD) * rD * (rt * rt);
+        const float R = k.h * (c.TF.h - t) -
+                        (lw.h + t2 * t2 * d3.h + c.d1u.h * (t - c.Taf.h) + c.d1i.h * (qs - c.aqh.h));
+        const float dF = 4.f * d3.h * t2 * t + c.d1u.h + c.d1i.h * dqs;
+        t = fminf(fmaxf(t + R * __frcp_rn(k.h + dF), gk.Tmin_f), gk.Tmelt_f);
     }
-    solve4temp_f64<NC, false>(p, gk, x, val(Tin), hIv, hSv, Tv, Fiov, Fiav, Penv);
-    const double aa1l2 = aa1 * 3.32192809488736234787;
-    const double qnum = bb1 * cc0, qsub = one_m_bb1 * cc0;
-#pragma unroll
-    for (int l = 0; l < NC; ++l) {
-        if (!ice[l]) {
-            oT[l] = Tin;
-            oFio[l] = S(0.0);
-            oFia[l] = S(0.0);
-            continue;
+    float dqs;
+    const Ff qs = saturation_ff(t, qnum, qsub, gk.cc1, dqs);
+    const float t2 = __fmul_rn(t, t);
+    const Ff tt = ff_fast_sum(t2, fmaf(t, t, -t2));
+    Ff Fc = ff_mul(k, ff_add(c.TF, -t));
+    Ff Fa = ff_add(ff_mul(ff_mul(tt, tt), d3), lw);
+    Fa = ff_add(Fa, ff_mul(c.d1u, ff_add(ff_neg(c.Taf), t)));
+    Fa = ff_add(Fa, ff_mul(c.d1i, ff_add(qs, ff_neg(c.aqh))));
+    const float res = (Fc.h - Fa.h) + (Fc.l - Fa.l);
+    const float dF = 4.f * d3.h * t2 * t + c.d1u.h + c.d1i.h * dqs;
+    const float step = res * __frcp_rn(k.h + dF);
+    const float tn = fminf(fmaxf(t + step, gk.Tmin_f), gk.Tmelt_f);
+    const double td = widen(t), Tmelt = p.celsius2K;
+    if (fabsf(tn - t) <= 4e-7f * t && fabsf(step) < 1e30f) {
+        T = td + widen(step);
+        float d = step;
+        if (gt64(T, Tmelt)) {
+            T = Tmelt;
+            d = narrow(Tmelt - td);
         }
-        const double t = Tv[l], t3 = t * t * t;
-        const double rt = 1.0 / t, c3 = ::exp2(aa1l2 * rt);
-        const double qs = qnum / (c3 * Pa - qsub), den = cc2 - c3 * Pa;
-        const double dqs = cc1 * c3 * (rt * rt) / (den * den);
-        const double FiaT = 4 * d3[l] * t3 + d1ug + d1iug * dqs;
-        const S Fc = k[l] * (x.TempFrz - t);
-        const S Fia = lwabs[l] + (t3 * t * d3[l] + d1ug * (t - Ta) + d1iug * (qs - x.aqh));
-        const bool held = t >= Tmelt || t <= Tmin;
-        S dT = Fc - Fia;   // its derivative part: R_theta
-        const double scale = held ? 0.0 : 1.0 / (val(k[l]) + FiaT);
-        S T = Tin, Fo = Fc, Fa = Fia;
-        T.v = t;
-#pragma unroll
-        for (int q = 0; q < (int)(sizeof(S::d) / sizeof(double)); ++q) {
-            const double dTq = dT.d[q] * scale;
-            T.d[q] = dTq;
-            Fo.d[q] = Fc.d[q] - val(k[l]) * dTq;
-            Fa.d[q] = Fia.d[q] + FiaT * dTq;
+        if (gt64(gk.Tmin, T)) {
+            T = gk.Tmin;
+            d = narrow(gk.Tmin - td);
         }
-        const bool up = Fiov[l] > 0;
-        Fo.v = Fiov[l];
-        Fa.v = Fiav[l];
-        oT[l] = T;
-        oFio[l] = up ? Fo : S(0.0);
-        oFia[l] = up ? S(0.0) : Fa;
+        if (!BARE) {
+            const float kd1 = __fmul_rn(k.h, d);
+            Fc = ff_add(Fc, Ff{-kd1, -(fmaf(k.h, d, -kd1) + k.l * d)});
+            Fa = ff_add(Fa, fmaf(6.f * d3.h * t2, d, dF) * d);
+            const bool up = Fc.h > 0.f;
+            const double F = ff_value(up ? Fc : Fa);
+            Fio = up ? F : 0.0;
+            Fia = up ? 0.0 : F;
+            if (root) {
+                root->up = up;
+                root->k = ff_value(k);
+                root->qs = ff_value(ff_add(qs, dqs * d));
+            }
+        }
+        return true;
+    }
+    // veris/solve4temp.py:108-160: six iterations and the fluxes at their end
+    const double qnumd = 0.622 * p.s4t_cc0, qsubd = (1.0 - 0.622) * p.s4t_cc0, d3d = emiss * p.stefBoltz;
+    if (NC == 5) kd = c.k0 / (double)(2 * l + 1);
+    double Fcd = 0.0, Fad = 0.0, qd = 0.0;
+    T = td;
+#pragma unroll 1
+    for (int it = 0; it < 7; ++it) {
+        const double rt = 1.0 / T, c3 = ::exp2(2663.5 * 3.32192809488736234787 * rt);
+        const double s2 = T * T, D = c3 * 100000.0 - qsubd, q = qnumd / D;
+        qd = q;
+        Fcd = kd * (x.TempFrz - T);
+        Fad = lwabs + s2 * s2 * d3d + c.d1ug * (T - c.Ta) + c.d1iug * (q - x.aqh);
+        if (it == 6) break;
+        const double Q = p.s4t_cc1 * c3 * (rt * rt) / (D * D);
+        T = T + (Fcd - Fad) / (kd + 4 * d3d * (s2 * T) + c.d1ug + c.d1iug * Q);
+        T = dmax(dmin(T, Tmelt), gk.Tmin);
+    }
+    const bool up = is_pos(Fcd);
+    if (!BARE) {
+        Fio = up ? Fcd : 0.0;
+        Fia = up ? 0.0 : Fad;
+        if (root) {
+            root->up = up;
+            root->k = kd;
+            root->qs = qd;
+        }
+    }
+    return finite64(up ? Fcd : Fad);
+}
+
+// the sums over the categories, hI (2l+1)/nITC and hS (2l+1)/nITC thick (veris/growth.py:62-92);
+// NC = 5, or 1 for any other number.
+// The loop stays rolled: unrolled it took 148 registers, 12 warps per SM, whose
+// latency bound the kernel (float64 pipe 43 % busy, 448 us on 1440 x 720); rolled
+// 317 us, and 265 with the kernel held to 80 registers, six CTAs per SM (four
+// 286, five 269, eight 269).
+template <int NC>
+__device__ __forceinline__ void solve4temp_sums(const VerisParams &p, const GrowthK &gk, const S4TIn &x, double Tin,
+                                                double hI, double hS, double &Tsum, double &Fio_sum, double &Fia_sum,
+                                                double &pen_sum) {
+    S4TCell c = solve4temp_cell<NC, false>(p, gk, x, Tin, hI * gk.pFac[0], hS * gk.pFac[0]);
+    const int n = NC == 5 ? 5 : p.nITC;
+#pragma unroll 1
+    for (int l = 0; l < n; ++l) {
+        double T = Tin, Fio = 0.0, Fia = 0.0, pen = 0.0;
+        const double f = NC == 5 ? gk.pFac[l] : (double)(2 * l + 1) * p.recip_nITC;
+        if (is_pos(hI) && is_pos(f))
+            solve4temp_category<NC, false>(p, gk, x, c, l, hI * f, hS * f, T, Fio, Fia, pen);
+        Tsum += T;
+        Fio_sum += Fio;
+        Fia_sum += Fia;
+        pen_sum += pen;
     }
 }
 
-template <int NC, class S>
-__device__ __forceinline__ void solve4temp_multi(const VerisParams &p, const GrowthK &gk, const S4TIn &x,
-                                                 const S &Tin, const S *hI, const S *hS, S *oT, S *oFio, S *oFia,
-                                                 S *oPen) {
-    if constexpr (std::is_same<S, double>::value) solve4temp_f64<NC, false>(p, gk, x, Tin, hI, hS, oT, oFio, oFia, oPen);
-    else solve4temp_dual<NC, S>(p, gk, x, Tin, hI, hS, oT, oFio, oFia, oPen);
-}
-
-template <class S>
 struct GrowthOut {
-    S h, hs, A, TSurf, EmPmR, forc_salt, Qsw, Qnet, load, pen, rh;
+    double h, hs, A, TSurf, EmPmR, forc_salt, Qsw, Qnet, load, pen, rh;
 };
 
 // sum / n < limit as IEEE division has it (all categories at the melting point
@@ -493,29 +424,28 @@ __device__ __forceinline__ bool mean_below(double sum, double n, double rn, doub
 
 // veris/growth.py:8-397 for one point, from the ice state (h, hs, A, TSurf)
 // and the forcing of point o
-template <class S>
-__device__ GrowthOut<S> growth_point(const VerisParams &p, const GrowthK &gk, const Fields<double> &f, int64_t o,
-                                     S hIn, S hsIn, S AIn, S TSurfIn) {
+__device__ __forceinline__ GrowthOut growth_point(const VerisParams &p, const GrowthK &gk, const Fields<double> &f, int64_t o,
+                                                 double hIn, double hsIn, double AIn, double TSurfIn) {
     const double qi = gk.qi;
     const double qs = gk.qs;
-    const bool noIce = vzero(hIn) || vzero(AIn);
-    S h0 = hIn, hs0 = hsIn, A0 = AIn;
+    const bool noIce = is_zero(hIn) || is_zero(AIn);
+    double h0 = hIn, hs0 = hsIn, A0 = AIn;
     if (noIce) {
         h0 = h0 * 0.0;
         hs0 = hs0 * 0.0;
         A0 = A0 * 0.0;
     }
-    const bool isIce = vpos(h0);
-    const S rregA = vrsqrt(A0 * A0 + p.Area_reg);
-    S hIa = isIce ? h0 * rregA : S(0.0);
-    const S rhIa = A0 * vrsqrt(h0 * h0 + p.hIce_reg);
-    const S hSa = isIce ? hs0 * rregA : S(0.0);
-    hIa = smax(hIa, S(0.05));
+    const bool isIce = is_pos(h0);
+    const double rregA = rsqrt_lane(A0 * A0 + p.Area_reg);
+    double hIa = isIce ? h0 * rregA : 0.0;
+    const double rhIa = A0 * rsqrt_lane(h0 * h0 + p.hIce_reg);
+    const double hSa = isIce ? hs0 * rregA : 0.0;
+    hIa = dmax(hIa, 0.05);
 
     const double ocSalt = __ldg(f.ocSalt + o);
     const double TempFrz = p.tempFrz + p.dtempFrz_dS * ocSalt + p.celsius2K;
     S4TIn x;
-    x.Tin = val(TSurfIn);
+    x.Tin = TSurfIn;
     x.TempFrz = TempFrz;
     x.LWdown = __ldg(f.LWdown + o);
     x.ATemp = __ldg(f.ATemp + o);
@@ -523,113 +453,89 @@ __device__ GrowthOut<S> growth_point(const VerisParams &p, const GrowthK &gk, co
     x.fCori = __ldg(f.fCori + o);
     x.SWdown = __ldg(f.SWdown + o);
     x.aqh = __ldg(f.aqh + o);
-    S Tsum = 0, Fio_sum = 0, Fia_sum = 0, pen_sum = 0;
-    if (p.nITC == 5) {
-        S hIc[5], hSc[5], rT[5], rFio[5], rFia[5], rPen[5];
-#pragma unroll
-        for (int l = 0; l < 5; ++l) {
-            hIc[l] = hIa * gk.pFac[l];
-            hSc[l] = hSa * gk.pFac[l];
-        }
-        solve4temp_multi<5, S>(p, gk, x, TSurfIn, hIc, hSc, rT, rFio, rFia, rPen);
-#pragma unroll
-        for (int l = 0; l < 5; ++l) {
-            Tsum = Tsum + rT[l];
-            Fio_sum = Fio_sum + rFio[l];
-            Fia_sum = Fia_sum + rFia[l];
-            pen_sum = pen_sum + rPen[l];
-        }
-    } else {
-        for (int l = 0; l < p.nITC; ++l) {
-            const double pFac = (double)(2 * (l + 1) - 1) * p.recip_nITC;
-            S hIc[1] = {hIa * pFac}, hSc[1] = {hSa * pFac}, rT[1], rFio[1], rFia[1], rPen[1];
-            solve4temp_multi<1, S>(p, gk, x, TSurfIn, hIc, hSc, rT, rFio, rFia, rPen);
-            Tsum = Tsum + rT[0];
-            Fio_sum = Fio_sum + rFio[0];
-            Fia_sum = Fia_sum + rFia[0];
-            pen_sum = pen_sum + rPen[0];
-        }
-    }
-    GrowthOut<S> g;
+    double Tsum = 0.0, Fio_sum = 0.0, Fia_sum = 0.0, pen_sum = 0.0;
+    if (p.nITC == 5) solve4temp_sums<5>(p, gk, x, TSurfIn, hIa, hSa, Tsum, Fio_sum, Fia_sum, pen_sum);
+    else solve4temp_sums<1>(p, gk, x, TSurfIn, hIa, hSa, Tsum, Fio_sum, Fia_sum, pen_sum);
+    GrowthOut g;
     g.TSurf = Tsum * p.recip_nITC;
-    const S An = A0 * p.recip_nITC;
-    const S Fio = Fio_sum * An;
-    S Fia = Fia_sum * An;
-    const S pen = pen_sum * An;
+    const double An = A0 * p.recip_nITC;
+    const double Fio = Fio_sum * An;
+    double Fia = Fia_sum * An;
+    const double pen = pen_sum * An;
 
     const double snowfall = __ldg(f.snowfall + o), precip = __ldg(f.precip + o);
-    const bool cold = vpos(A0) && mean_below(val(Tsum), gk.n, gk.rn, p.celsius2K);
+    const bool cold = is_pos(A0) && mean_below(Tsum, gk.n, gk.rn, p.celsius2K);
     const double snowAcc = (cold ? snowfall + precip : snowfall) * p.rhoFresh2rhoSnow;
     const double rainToSea = cold ? 0.0 : precip;
-    const S snowAccOverIce = snowAcc * A0 * p.deltatTherm;
+    const double snowAccOverIce = snowAcc * A0 * p.deltatTherm;
 
-    S gUnder = Fio * qi;
-    if (vzero(A0)) gUnder = S(0.0);
-    const S potMeltRate = -Fia * qs;
-    const S potMelt = potMeltRate * p.deltatTherm;
-    const bool allMelt = vge(potMelt, hs0);
-    const S meltRate = allMelt ? hs0 * p.recip_deltatTherm : potMeltRate;
-    const S toSnow = allMelt ? -hs0 * p.recip_deltatTherm * gk.rqs : Fia;
+    double gUnder = Fio * qi;
+    if (is_zero(A0)) gUnder = 0.0;
+    const double potMeltRate = -Fia * qs;
+    const double potMelt = potMeltRate * p.deltatTherm;
+    const bool allMelt = ge64(potMelt, hs0);
+    const double meltRate = allMelt ? hs0 * p.recip_deltatTherm : potMeltRate;
+    const double toSnow = allMelt ? -hs0 * p.recip_deltatTherm * gk.rqs : Fia;
     Fia = Fia - toSnow;
-    const S gSurf = Fia * qi;
-    const S gNet = (gUnder + gSurf) * rregA;
+    const double gSurf = Fia * qi;
+    const double gNet = (gUnder + gSurf) * rregA;
 
     const double t0 = 0.4, t1 = 7 / t0;
     const double t2 = gk.t2;
     const double sst = dmax(__ldg(f.theta + o), TempFrz);
-    const S mltf = 1 + vdiv(p.McPheeTaperFac - 1, 1 + vexp((A0 - t0) * t1));
-    const S gML = -t2 * (sst - TempFrz) * mltf * qi;
+    const double mltf = 1 + div_lane(p.McPheeTaperFac - 1, 1 + exp_table((A0 - t0) * t1));
+    const double gML = -t2 * (sst - TempFrz) * mltf * qi;
     const double Qnet_in = __ldg(f.Qnet + o);
     const double gOW = qi * Qnet_in;
 
-    const S dh = gNet * A0 + gOW * (1 - A0) + gML;
-    const S dhs = (snowAcc - meltRate) * A0;
-    const S half_rh = 0.5 * rhIa;
-    S dA_oa = half_rh * gOW * (1 - A0);
-    const bool grow = is_pos(gOW) && (vpos(A0) || vpos(dh));
+    const double dh = gNet * A0 + gOW * (1 - A0) + gML;
+    const double dhs = (snowAcc - meltRate) * A0;
+    const double half_rh = 0.5 * rhIa;
+    double dA_oa = half_rh * gOW * (1 - A0);
+    const bool grow = is_pos(gOW) && (is_pos(A0) || is_pos(dh));
     if (grow) dA_oa = gOW * (1 - A0);
     const double fC = __ldg(f.fCori + o);
     dA_oa = (grow && is_neg(fC)) ? dA_oa * p.recip_h0_south : dA_oa * p.recip_h0;
-    const S dA_oi = vle0(gML) ? half_rh * gML : S(0.0);
-    const S dA_ia = (vle0(gNet) && vpos(h0)) ? half_rh * gNet * A0 : S(0.0);
-    const S dA = dA_oa + dA_oi + dA_ia;
+    const double dA_oi = !is_pos(gML) && !is_nan64(gML) ? half_rh * gML : 0.0;
+    const double dA_ia = (!is_pos(gNet) && !is_nan64(gNet) && is_pos(h0)) ? half_rh * gNet * A0 : 0.0;
+    const double dA = dA_oa + dA_oi + dA_ia;
 
     const double mask = __ldg(f.iceMask + o);
     const double mdt = mask * p.deltatTherm;
-    S A = A0 + dA * mdt;
-    S h = h0 + dh * mdt;
-    S hs = hs0 + dhs * mdt;
-    A = smin(smax(A, S(0.0)), S(1.0));
-    h = smax(h, S(0.0));
-    hs = smax(hs, S(0.0));
-    if (vzero(h) || vzero(A)) {
+    double A = A0 + dA * mdt;
+    double h = h0 + dh * mdt;
+    double hs = hs0 + dhs * mdt;
+    A = dmin(dmax(A, 0.0), 1.0);
+    h = dmax(h, 0.0);
+    hs = dmax(hs, 0.0);
+    if (is_zero(h) || is_zero(A)) {
         A = A * 0.0;
         hs = hs * 0.0;
         h = h * 0.0;
     }
-    const S hsub = (hs * p.rhoSnow + h * p.rhoIce) * p.recip_rhoSea;
-    const S flood = smax(S(0.0), hsub - h);
+    const double hsub = (hs * p.rhoSnow + h * p.rhoIce) * p.recip_rhoSea;
+    const double flood = dmax(0.0, hsub - h);
     h = h + flood;
     hs = hs - flood * p.rhoIce2rhoSnow;
-    g.rh = vrsqrt(h * h + p.hIce_reg);
+    g.rh = rsqrt_lane(h * h + p.hIce_reg);
     g.h = h;
     g.hs = hs;
     g.A = A;
 
     g.Qsw = pen * A0 + __ldg(f.Qsw + o) * (1 - A0);
-    const S dH = h - h0;
-    const S melted = hs0 + snowAccOverIce - hs;
-    const S E_ice = dH * gk.rqi;
-    const S E_out = (A0 * (Fia + Fio + pen) + (1 - A0) * Qnet_in) * p.deltatTherm;
+    const double dH = h - h0;
+    const double melted = hs0 + snowAccOverIce - hs;
+    const double E_ice = dH * gk.rqi;
+    const double E_out = (A0 * (Fia + Fio + pen) + (1 - A0) * Qnet_in) * p.deltatTherm;
     g.Qnet = (E_out - E_ice) * p.recip_deltatTherm;
-    S fw_ice = -dH * p.rhoIce2rhoFresh;
+    double fw_ice = -dH * p.rhoIce2rhoFresh;
     if (p.saltIce_ref != 0.0 && is_pos(ocSalt) && gt64(ocSalt, p.saltIce_ref))
         fw_ice = fw_ice * (1 - p.saltIce_ref / ocSalt);
     const double salt_ref = dmin(p.saltIce_ref, ocSalt);
     const double osh = __ldg(f.os_hIceMean + o), oshs = __ldg(f.os_hSnowMean + o);
-    S saltflux = S(0.0);
+    double saltflux = 0.0;
     if (!is_zero(salt_ref)) saltflux = (dH + osh) * salt_ref * mask * p.rhoIce * p.recip_deltatTherm;
-    const S fw_snow = melted * gk.rf2s;
+    const double fw_snow = melted * gk.rf2s;
     g.EmPmR = mask * ((-__ldg(f.evap + o) - precip) * (1 - A0) - rainToSea * A0 - __ldg(f.runoff + o) -
                       (fw_ice + fw_snow) * p.recip_deltatTherm) * p.rhoFresh +
               mask * (osh * p.rhoIce + oshs * p.rhoSnow) * p.recip_deltatTherm;
@@ -673,7 +579,7 @@ struct GrowthPtrs {
 // general point's float64 operations.  False where an input that the reference
 // multiplies by zero is not finite (the caller takes the general point).
 __device__ __forceinline__ bool growth_bare(const VerisParams &p, const GrowthK &gk, const Fields<double> &f,
-                                            int64_t o, unsigned m, double TSurfIn, GrowthOut<double> &g) {
+                                            int64_t o, unsigned m, double TSurfIn, GrowthOut &g) {
     const double ocSalt = __ldg(f.ocSalt + o), fC = __ldg(f.fCori + o);
     S4TIn x;
     x.TempFrz = p.tempFrz + p.dtempFrz_dS * ocSalt + p.celsius2K;
@@ -683,12 +589,18 @@ __device__ __forceinline__ bool growth_bare(const VerisParams &p, const GrowthK 
     x.fCori = fC;
     x.SWdown = __ldg(f.SWdown + o);
     x.aqh = __ldg(f.aqh + o);
-    const double none[1] = {0.0};
-    double T[5];
-    const bool finite = solve4temp_f64<5, true>(p, gk, x, TSurfIn, none, none, T, nullptr, nullptr, nullptr);
+    S4TCell c = solve4temp_cell<5, true>(p, gk, x, TSurfIn, 0.0, 0.0);
+    double Tsum = 0.0;
+    bool finite = true;
+#pragma unroll 1
+    for (int l = 0; l < 5; ++l) {
+        double T, unused0, unused1, unused2;
+        finite = solve4temp_category<5, true>(p, gk, x, c, l, 0.0, 0.0, T, unused0, unused1, unused2) && finite;
+        Tsum += T;
+    }
     const double snowfall = __ldg(f.snowfall + o), precip = __ldg(f.precip + o);
     if (!__all_sync(m, finite && finite64(snowfall) && finite64(precip))) return false;
-    g.TSurf = ((((T[0] + T[1]) + T[2]) + T[3]) + T[4]) * p.recip_nITC;
+    g.TSurf = Tsum * p.recip_nITC;
     const double Qnet = __ldg(f.Qnet + o), mask = __ldg(f.iceMask + o);
     const double gOW = gk.qi * Qnet;
     const double dh = gOW + gk.meltb * (dmax(__ldg(f.theta + o), x.TempFrz) - x.TempFrz);
@@ -730,7 +642,7 @@ __device__ __forceinline__ bool growth_bare(const VerisParams &p, const GrowthK 
 }
 
 // rows [i0, i1) of the padded array (Growth is pointwise)
-__global__ void __launch_bounds__(128) growth_kernel(VerisParams p, GrowthK gk, Fields<double> f, Dims d,
+__global__ void __launch_bounds__(128, 6) growth_kernel(VerisParams p, GrowthK gk, Fields<double> f, Dims d,
                                                      GrowthPtrs out, int i0, int i1) {
     const int j = blockIdx.x * 32 + threadIdx.x, i = i0 + blockIdx.y * 4 + threadIdx.y;
     const unsigned m = __ballot_sync(0xffffffffu, i < i1 && j < d.NY);
@@ -738,10 +650,10 @@ __global__ void __launch_bounds__(128) growth_kernel(VerisParams p, GrowthK gk, 
     const int64_t o = d.raw(i, j);
     const double h0 = __ldg(f.hIceMean + o), hs0 = __ldg(f.hSnowMean + o), A0 = __ldg(f.Area + o);
     const double T0 = __ldg(f.TSurf + o);
-    GrowthOut<double> g;
+    GrowthOut g;
     const bool water = p.nITC == 5 && (is_zero(h0) || is_zero(A0)) && finite64(h0) && finite64(hs0) && finite64(A0);
     if (!(__all_sync(m, water) && growth_bare(p, gk, f, o, m, T0, g)))
-        g = growth_point<double>(p, gk, f, o, h0, hs0, A0, T0);
+        g = growth_point(p, gk, f, o, h0, hs0, A0, T0);
     out.h[o] = g.h;
     out.hs[o] = g.hs;
     out.A[o] = g.A;
@@ -755,25 +667,189 @@ __global__ void __launch_bounds__(128) growth_kernel(VerisParams p, GrowthK gk, 
     out.rh[o] = g.rh;
 }
 
-// adjoint of growth for the ice state: l_in = J^T l_out over (h, hs, A, TSurf)
-__global__ void __launch_bounds__(128) growth_adjoint_kernel(VerisParams p, GrowthK gk, Fields<double> f, Dims d,
+// Adjoint of growth_point for the ice state (h, hs, A): given the adjoints of
+// the new h, hs, A and TSurf, one forward pass for the values and one reverse
+// pass (branches as in the forward).  TSurf enters Growth as the first guess
+// of a converged iteration only: its adjoint is 0.
+//
+// solve4temp's categories: at the root T of R(T) = Fc(T) - Fia(T),
+// dT = -R_theta / R_T with R_theta the residual's derivative at fixed T
+// (through the conductivity k and the absorbed shortwave) and R_T =
+// -(k + dFia/dT), the Newton iteration's own denominator; a root held by the
+// melt or the minimum-temperature clamp has dT = 0.  (The converged Newton
+// iterates have this derivative.)  Each category's shares in the adjoints of
+// the ice and snow thickness are linear in the adjoints of the summed T, Fio
+// and Fia, the last two known only after the sums, so the one loop collects
+// the six coefficients (Q: through k, W: through the shortwave).
+//
+// 721 x 359 points: dual numbers for four inputs took 1.05 ms (1455 float64
+// operations per point); this, with open water skipped, 0.23 ms (four CTAs per SM;
+// six 0.24).
+template <int NC>
+__device__ __forceinline__ void growth_adjoint_point(const VerisParams &p, const GrowthK &gk,
+                                                     const Fields<double> &f, int64_t o, double h0, double hs0,
+                                                     double A0, double Tin, double l_h, double l_hs, double l_A,
+                                                     double l_T, double &a_h, double &a_hs, double &a_A) {
+    const bool isIce = is_pos(h0);
+    const double rregA = rsqrt_lane(A0 * A0 + p.Area_reg), rregh = rsqrt_lane(h0 * h0 + p.hIce_reg);
+    const double hIreg = isIce ? h0 * rregA : 0.0, hSa = isIce ? hs0 * rregA : 0.0;
+    const bool thick = gt64(hIreg, 0.05);
+    const double hIa = thick ? hIreg : 0.05;
+    S4TIn x;
+    x.TempFrz = p.tempFrz + p.dtempFrz_dS * __ldg(f.ocSalt + o) + p.celsius2K;
+    x.LWdown = __ldg(f.LWdown + o);
+    x.ATemp = __ldg(f.ATemp + o);
+    x.wSpeed = __ldg(f.wSpeed + o);
+    x.fCori = __ldg(f.fCori + o);
+    x.SWdown = __ldg(f.SWdown + o);
+    x.aqh = __ldg(f.aqh + o);
+
+    // ---- the categories: sums, and the coefficients of their adjoints
+    double Tsum = 0.0, Fio_sum = 0.0, Fia_sum = 0.0;
+    double QT = 0.0, Qio = 0.0, Qia = 0.0, WT = 0.0, Wio = 0.0, Wia = 0.0;
+    {
+        S4TCell c = solve4temp_cell<NC, false>(p, gk, x, Tin, hIa * gk.pFac[0], hSa * gk.pFac[0]);
+        const int n = NC == 5 ? 5 : p.nITC;
+#pragma unroll 1
+        for (int l = 0; l < n; ++l) {
+            double T = Tin, Fio = 0.0, Fia = 0.0, pen;
+            const double fl = NC == 5 ? gk.pFac[l] : (double)(2 * l + 1) * p.recip_nITC;
+            if (is_pos(fl)) {
+                S4TRoot r;
+                solve4temp_category<NC, false>(p, gk, x, c, l, hIa * fl, hSa * fl, T, Fio, Fia, pen, &r);
+                const double d3 = (is_pos(hSa * fl) ? p.snowEmiss : p.iceEmiss) * p.stefBoltz;
+                const double T2 = T * T;
+                // d qs / dT = qs (1 + qs qsub/qnum) aa1 ln10 / T^2
+                const double dqs = r.qs * fma(r.qs, gk.qratio, 1.0) * (gk.aln10 * rcp_lane(T2));
+                const double FiaT = fma(c.d1iug, dqs, fma(4.0 * d3, T2 * T, c.d1ug));
+                const bool held = ge64(T, p.celsius2K) || ge64(gk.Tmin, T);
+                const double s = held ? 0.0 : rcp_lane(r.k + FiaT);
+                const double ks = r.k * s, fs = FiaT * s;
+                const double u = r.k * r.k * fl * (x.TempFrz - T), w = r.dSW * fl;
+                QT = fma(u, s, QT);
+                WT = fma(w, s, WT);
+                if (r.up) {
+                    Qio = fma(u, held ? 1.0 : fs, Qio);
+                    Wio = fma(-w, ks, Wio);
+                } else {
+                    Qia = fma(u, fs, Qia);
+                    Wia = fma(-w, held ? 1.0 : ks, Wia);
+                }
+            }
+            Tsum += T;
+            Fio_sum += Fio;
+            Fia_sum += Fia;
+        }
+    }
+
+    // ---- forward (growth_point)
+    const double An = A0 * p.recip_nITC, Fio = Fio_sum * An, Fia = Fia_sum * An;
+    const bool cold = is_pos(A0) && mean_below(Tsum, gk.n, gk.rn, p.celsius2K);
+    const double snowfall = __ldg(f.snowfall + o), precip = __ldg(f.precip + o);
+    const double snowAcc = (cold ? snowfall + precip : snowfall) * p.rhoFresh2rhoSnow;
+    const double potMeltRate = -Fia * gk.qs;
+    const bool allMelt = ge64(potMeltRate * p.deltatTherm, hs0);
+    const double meltRate = allMelt ? hs0 * p.recip_deltatTherm : potMeltRate;
+    const double FiaR = allMelt ? Fia + hs0 * p.recip_deltatTherm * gk.rqs : 0.0;   // what melts ice
+    const double G = ((is_zero(A0) ? 0.0 : Fio) + FiaR) * gk.qi;
+    const double gNet = G * rregA;
+    const double t0 = 0.4, t1 = 7 / t0;
+    const double E = exp_table((A0 - t0) * t1), rE = rcp_lane(1.0 + E);
+    const double M = p.McPheeTaperFac - 1;
+    const double cML = -gk.t2 * (dmax(__ldg(f.theta + o), x.TempFrz) - x.TempFrz) * gk.qi;
+    const double gML = cML * fma(M, rE, 1.0);
+    const double gOW = gk.qi * __ldg(f.Qnet + o), open = 1.0 - A0;
+    const double dh = gNet * A0 + gOW * open + gML;
+    const double half = 0.5 * A0 * rregh;
+    const bool grow = is_pos(gOW) && (is_pos(A0) || is_pos(dh));
+    const double rh0 = (grow && is_neg(x.fCori)) ? p.recip_h0_south : p.recip_h0;
+    const bool melts = !is_pos(gML) && !is_nan64(gML), thins = !is_pos(gNet) && !is_nan64(gNet) && isIce;
+    const double dA_oa = (grow ? gOW : half * gOW) * open * rh0;
+    const double dA = dA_oa + (melts ? half * gML : 0.0) + (thins ? half * gNet * A0 : 0.0);
+    const double mdt = __ldg(f.iceMask + o) * p.deltatTherm;
+    const double A1 = A0 + dA * mdt, h1 = h0 + dh * mdt, hs1 = hs0 + (snowAcc - meltRate) * A0 * mdt;
+    const bool keepA = is_pos(A1) && gt64(1.0, A1), keeph = is_pos(h1), keephs = is_pos(hs1);
+
+    // ---- reverse: flooding, the clips, the increments
+    double gh = l_h, ghs = l_hs, gA = l_A;
+    const double hc = keeph ? h1 : 0.0, hsc = keephs ? hs1 : 0.0;
+    if (!gt64(0.0, (hsc * p.rhoSnow + hc * p.rhoIce) * p.recip_rhoSea - hc)) {
+        const double gf = l_h - l_hs * p.rhoIce2rhoSnow;
+        gh = fma(gf, p.rhoIce * p.recip_rhoSea - 1.0, gh);
+        ghs = fma(gf, p.rhoSnow * p.recip_rhoSea, ghs);
+    }
+    if (!keeph || !is_pos(A1)) gh = ghs = gA = 0.0;   // no ice left
+    if (!keephs) ghs = 0.0;
+    if (!keepA) gA = 0.0;
+    const double gdA = gA * mdt, gdh = gh * mdt, gdhs = ghs * mdt;
+    const double g_melt = -gdhs * A0;
+    double g_A = fma(gdhs, snowAcc - meltRate, gA);
+    g_A = fma(gdh, gNet - gOW, g_A);
+    double g_hs = ghs, g_h = gh;
+    double g_gNet = gdh * A0, g_gML = gdh, g_half = 0.0;
+    g_A = fma(-gdA * rh0, grow ? gOW : half * gOW, g_A);
+    if (!grow) g_half = gdA * gOW * open * rh0;
+    if (melts) {
+        g_half = fma(gdA, gML, g_half);
+        g_gML = fma(gdA, half, g_gML);
+    }
+    if (thins) {
+        g_half = fma(gdA, gNet * A0, g_half);
+        g_gNet = fma(gdA, half * A0, g_gNet);
+        g_A = fma(gdA, half * gNet, g_A);
+    }
+    const double g_rhI = 0.5 * g_half * rregh;   // rhIa = A0 / sqrt(h0^2 + reg)
+    g_A += g_rhI;
+    g_h = fma(-g_rhI * A0 * h0, rregh * rregh, g_h);
+    g_A = fma(-g_gML * cML * M * t1 * E, rE * rE, g_A);
+    // ---- the fluxes
+    const double g_G = g_gNet * rregA * gk.qi;   // per W/m2
+    double g_rregA = g_gNet * G, g_Fio = is_zero(A0) ? 0.0 : g_G, g_Fia;
+    if (allMelt) {
+        g_Fia = g_G;
+        g_hs = fma(fma(g_G, gk.rqs, g_melt), p.recip_deltatTherm, g_hs);
+    } else {
+        g_Fia = -gk.qs * g_melt;
+    }
+    g_A = fma(fma(g_Fio, Fio_sum, g_Fia * Fia_sum), p.recip_nITC, g_A);
+    const double sT = l_T * p.recip_nITC, sio = g_Fio * An, sia = g_Fia * An;
+    const double Q = -(QT * sT + Qio * sio + Qia * sia) * gk.rkk, W = WT * sT + Wio * sio + Wia * sia;
+    double g_hI = Q * p.snowConduct, g_hS = Q * p.iceConduct;
+    if (is_pos(hSa)) g_hS += W;
+    else g_hI += W;
+    if (!thick) g_hI = 0.0;
+    if (isIce) {   // hIa = h0 rregA, hSa = hs0 rregA
+        g_h = fma(g_hI, rregA, g_h);
+        g_hs = fma(g_hS, rregA, g_hs);
+        g_rregA = fma(g_hI, h0, fma(g_hS, hs0, g_rregA));
+    }
+    a_A = fma(-g_rregA * A0 * rregA, rregA * rregA, g_A);
+    a_h = g_h;
+    a_hs = g_hs;
+}
+
+__global__ void __launch_bounds__(128, 4) growth_adjoint_kernel(VerisParams p, GrowthK gk, Fields<double> f, Dims d,
                                                              const double *lh, const double *lhs, const double *lA,
                                                              const double *lT, double *oh, double *ohs, double *oA,
                                                              double *oT) {
     const int j = blockIdx.x * 32 + threadIdx.x, i = blockIdx.y * 4 + threadIdx.y;
     if (i >= d.NX || j >= d.NY) return;
     const int64_t o = d.raw(i, j);
-    using D = Dual<4>;
-    const GrowthOut<D> g = growth_point<D>(p, gk, f, o, D::var(f.hIceMean[o], 0), D::var(f.hSnowMean[o], 1),
-                                           D::var(f.Area[o], 2), D::var(f.TSurf[o], 3));
+    const double h0 = __ldg(f.hIceMean + o), hs0 = __ldg(f.hSnowMean + o), A0 = __ldg(f.Area + o);
     const double l0 = lh[o], l1 = lhs[o], l2 = lA[o], l3 = lT[o];
-    double r[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) r[k] = l0 * g.h.d[k] + l1 * g.hs.d[k] + l2 * g.A.d[k] + l3 * g.TSurf.d[k];
-    oh[o] = r[0];
-    ohs[o] = r[1];
-    oA[o] = r[2];
-    oT[o] = r[3];
+    double a_h = 0.0, a_hs = 0.0, a_A = 0.0;
+    if (is_zero(h0) || is_zero(A0)) {   // Growth multiplies the three by zero there
+        a_h = (l0 + l1 + l2 + l3) * 0.0;
+        a_hs = a_A = a_h;
+    } else if (p.nITC == 5) {
+        growth_adjoint_point<5>(p, gk, f, o, h0, hs0, A0, __ldg(f.TSurf + o), l0, l1, l2, l3, a_h, a_hs, a_A);
+    } else {
+        growth_adjoint_point<1>(p, gk, f, o, h0, hs0, A0, __ldg(f.TSurf + o), l0, l1, l2, l3, a_h, a_hs, a_A);
+    }
+    oh[o] = a_h;
+    ohs[o] = a_hs;
+    oA[o] = a_A;
+    oT[o] = (l0 + l1 + l2 + l3) * 0.0;
 }
 
 }  // namespace veris
