@@ -5,7 +5,9 @@
 // Dimensionally split: zonal fluxes, zonal update, meridional fluxes (of the
 // zonally updated field), meridional update.  Each phase is one launch over
 // all advected fields (blockIdx.z = field).  The fluxes are stored with the
-// halo fill the reference applies to them fused into the store.
+// halo fill the reference applies to them fused into the store.  (Float64
+// runs advection64.cu.)
+#include "advection64.cuh"
 #include "stencil.cuh"
 #include "dual.cuh"
 
@@ -369,6 +371,17 @@ static int advect(const VerisGrid *g, const VerisParams *p, const Fields<T> *vs,
         io.G[q] = reinterpret_cast<T *>(w + (2 + 2 * MAX_ADV_FIELDS + q) * fb);
     }
     cudaStream_t st = (cudaStream_t)s;
+    if constexpr (sizeof(T) == 8) {   // the passes below: a limiter bound under 2, very long grids
+        if (advect64_covers(*p, d)) {
+            Adv64IO io64;
+            for (int q = 0; q < MAX_ADV_FIELDS; ++q) {
+                io64.field[q] = io.field[q];
+                io64.f1[q] = io.f1[q];
+                io64.out[q] = io.out[q];
+            }
+            return advect64(c, h, io64, nf, st);
+        }
+    }
     dim3 bl(ABX, ABY);
     dim3 g2((d.NY + ABX - 1) / ABX, (d.NX + ABY - 1) / ABY);
     dim3 g3(g2.x, g2.y, nf);
