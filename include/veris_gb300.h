@@ -295,6 +295,10 @@ int veris_evp_fast_settings_check(const VerisParams *p);
 int veris_evp_walk_settings_check(const VerisParams *p);
 int veris_evp_fast_check(const VerisGrid *g, const VerisParams *p, const VerisFieldsF64 *vs,
                          int32_t *violations_device, veris_stream_t s);
+/* bit 128 alone (reads four fields): what the walk asks of a state that is
+ * otherwise known to be inside the fast form */
+int veris_evp_area_check(const VerisGrid *g, const VerisParams *p, const VerisFieldsF64 *vs,
+                         int32_t *violations_device, veris_stream_t s);
 int veris_evp_fast_solver_f32(const VerisGrid *g, const VerisParams *p, const VerisFieldsF64 *vs,
                               int32_t n_subcycles, float *uIce, float *vIce, float *sigma1,
                               float *sigma2, float *sigma12, void *workspace,

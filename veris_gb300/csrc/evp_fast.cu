@@ -23,6 +23,7 @@
 // masks 0/1, 1-D grid lengths); veris_evp_fast_check reports what a state
 // breaks, and callers use the plain form for those.
 #include "evp_tile.cuh"
+#include "f64math.cuh"
 
 namespace veris {
 
@@ -36,31 +37,57 @@ int fast_support(const VerisParams &p) {
 }
 
 // ------------------------------------------------------------------ checks
+// the cell areas' part: all the register walk asks of a state that the caller
+// knows to be the host model's
+__device__ __forceinline__ int area_violations(const Fields<double> &f, int64_t o, int64_t oj) {
+    return ne64(f.recip_rA[o], f.recip_rA[oj]) || ne64(f.rAz[o], f.rAz[oj]) || ne64(f.recip_rAu[o], f.recip_rAu[oj]) ||
+                   ne64(f.recip_rAv[o], f.recip_rAv[oj])
+               ? V_AREA2D
+               : 0;
+}
+
+// Comparisons on the integer pipe: as float64 comparisons, 28 per cell, they
+// bound the check (163 us on 2400 x 1200; its reads take 75).
 __global__ void fast_check_kernel(Fields<double> f, Dims d, int *viol) {
     const int j = blockIdx.x * 32 + threadIdx.x, i = blockIdx.y * 8 + threadIdx.y;
     if (i >= d.NX || j >= d.NY) return;
     const int64_t o = d.raw(i, j), o0 = d.raw(i, 0), oj = d.raw(0, j);
-    int v = 0;
-    if (f.k1AtC[o] != 0.0 || f.k2AtC[o] != 0.0 || f.k1AtZ[o] != 0.0 || f.k2AtZ[o] != 0.0) v |= V_KTERMS;
+    int v = area_violations(f, o, oj);
+    if (!is_zero(f.k1AtC[o]) || !is_zero(f.k2AtC[o]) || !is_zero(f.k1AtZ[o]) || !is_zero(f.k2AtZ[o])) v |= V_KTERMS;
     const double *m[6] = {f.iceMask, f.iceMaskU, f.iceMaskV, f.maskInC, f.maskInU, f.maskInV};
     for (int q = 0; q < 6; ++q)
-        if (m[q][o] != 0.0 && m[q][o] != 1.0) v |= V_MASKS;
-    if (f.recip_dxU[o] != f.recip_dxU[o0] || f.recip_dxV[o] != f.recip_dxV[o0] || f.dxV[o] != f.dxV[o0] ||
-        f.dxU[o] != f.dxU[o0])
+        if (!is_zero(m[q][o]) && ne64(m[q][o], 1.0)) v |= V_MASKS;
+    if (ne64(f.recip_dxU[o], f.recip_dxU[o0]) || ne64(f.recip_dxV[o], f.recip_dxV[o0]) || ne64(f.dxV[o], f.dxV[o0]) ||
+        ne64(f.dxU[o], f.dxU[o0]))
         v |= V_METRIC;
-    if (f.recip_dyV[o] != f.recip_dyV[oj] || f.recip_dyU[o] != f.recip_dyU[oj] || f.dyV[o] != f.dyV[oj] ||
-        f.dyU[o] != f.dyU[oj])
+    if (ne64(f.recip_dyV[o], f.recip_dyV[oj]) || ne64(f.recip_dyU[o], f.recip_dyU[oj]) ||
+        ne64(f.dyV[o], f.dyV[oj]) || ne64(f.dyU[o], f.dyU[oj]))
         v |= V_METRIC;
-    if (f.recip_rA[o] != f.recip_rA[oj] || f.rAz[o] != f.rAz[oj] || f.recip_rAu[o] != f.recip_rAu[oj] ||
-        f.recip_rAv[o] != f.recip_rAv[oj])
-        v |= V_AREA2D;
+    if (v) atomicOr(viol, v);
+}
+
+__global__ void area_check_kernel(Fields<double> f, Dims d, int *viol) {
+    const int j = blockIdx.x * 32 + threadIdx.x, i = blockIdx.y * 8 + threadIdx.y;
+    if (i >= d.NX || j >= d.NY) return;
+    const int v = area_violations(f, d.raw(i, j), d.raw(0, j));
     if (v) atomicOr(viol, v);
 }
 
 // ------------------------------------------------------------------- prep
+// the basal drag's step factor (veris/dynamics_routines.py:65-94)
+__device__ __forceinline__ double basal_factor(const VerisParams &p, const Fields<double> &f, int64_t o) {
+    const double A = f.Area[o];
+    double b = 0.0;
+    if (A > 0.01) {
+        const double hcrit = fabs(f.R_low[o]) * A / p.basalDragK1;
+        b = p.basalDragK2 * log(exp(10.0 * (f.hIceMean[o] - hcrit)) + 1.0) * 0.1 * exp(-p.cBasalStar * (1.0 - A));
+    }
+    return b;
+}
+
 template <class T, bool BASAL>
 __global__ void fast_prep_kernel(VerisParams p, Fields<double> f, Dims d, int64_t lp, FastConsts<T> c, T *u, T *v,
-                                 T *s1, T *s2, T *s12, int paired) {
+                                 T *s1, T *s2, T *s12) {
     const int j = blockIdx.x * 32 + threadIdx.x, i = blockIdx.y * 8 + threadIdx.y;
     if (i >= d.NX || j >= d.NY) return;
     const int64_t o = d.raw(i, j);
@@ -123,14 +150,7 @@ __global__ void fast_prep_kernel(VerisParams p, Fields<double> f, Dims d, int64_
         }
     }
     if (BASAL) {
-        const double A = f.Area[o];
-        double b = 0.0;
-        if (A > 0.01) {
-            const double hcrit = fabs(f.R_low[o]) * A / p.basalDragK1;
-            b = p.basalDragK2 * log(exp(10.0 * (f.hIceMean[o] - hcrit)) + 1.0) * 0.1 *
-                exp(-p.cBasalStar * (1.0 - A));
-        }
-        c.bfac[q] = (T)b;
+        c.bfac[q] = (T)basal_factor(p, f, o);
     }
     const double fc = f.fCori[o];
     uint32_t fl = 0;
@@ -167,18 +187,70 @@ __global__ void fast_prep_kernel(VerisParams p, Fields<double> f, Dims d, int64_
         c.rrAu_y[j] = (T)f.recip_rAu[o];
         c.rrAv_y[j] = (T)f.recip_rAv[o];
     }
-    if (paired) {   // the register walk's layout: (u, v, sigma1, sigma2) over the four buffers
-        u[4 * q] = (T)f.uIce[o];
-        u[4 * q + 1] = (T)f.vIce[o];
-        u[4 * q + 2] = (T)f.sigma1[o];
-        u[4 * q + 3] = (T)f.sigma2[o];
-    } else {
-        u[q] = (T)f.uIce[o];
-        v[q] = (T)f.vIce[o];
-        s1[q] = (T)f.sigma1[o];
-        s2[q] = (T)f.sigma2[o];
-    }
+    u[q] = (T)f.uIce[o];
+    v[q] = (T)f.vIce[o];
+    s1[q] = (T)f.sigma1[o];
+    s2[q] = (T)f.sigma2[o];
     s12[q] = (T)f.sigma12[o];
+}
+
+// The register walk's part of the fold, for a walk that takes the cell areas
+// along j: the four 16- and 8-byte groups it reads, its state and flags, each
+// in one store (fast_prep_kernel writes them by components, 16 bytes apart,
+// and the planar copies of the other forms beside them), float32 conversions
+// on the integer pipe.  Bound by the 26 float64 reads: 2400 x 1200 311 -> 125 us.
+template <bool BASAL>
+__global__ void walk_prep_kernel(const __grid_constant__ Ctx<double> x, int64_t lp, FastConsts<float> c, float4 *state,
+                                 float *s12) {
+    const int j = blockIdx.x * 32 + threadIdx.x, i = blockIdx.y * 8 + threadIdx.y;
+    const Dims &d = x.d;
+    const VerisParams &p = x.p;
+    const Fields<double> &f = x.f;
+    if (i >= d.NX || j >= d.NY) return;
+    const int64_t o = d.raw(i, j);
+    const int64_t q = (int64_t)i * lp + j;
+    const double rdt = p.recip_deltatDyn;
+    const double P = f.SeaIceStrength[o];
+    const double mC = f.SeaIceMassC[o], fc = f.fCori[o], mU = f.SeaIceMassU[o], mV = f.SeaIceMassV[o];
+    const double u = f.uIce[o], v = f.vIce[o];
+    state[q] = make_float4(to_float(u), to_float(v), to_float(f.sigma1[o]), to_float(f.sigma2[o]));
+    s12[q] = to_float(f.sigma12[o]);
+    reinterpret_cast<float4 *>(c.q4O)[q] =
+        make_float4(to_float(f.uOcean[o]), to_float(f.vOcean[o]), to_float(mC * fc * 0.5),
+                    to_float(0.5 * P * (1.0 + p.tensileStrFac)));
+    reinterpret_cast<float4 *>(c.q4U)[q] =
+        make_float4(to_float(mU * rdt * u + f.WindForcingX[o]), to_float(mV * rdt * v + f.WindForcingY[o]),
+                    to_float(f.AreaW[o]), to_float(f.AreaS[o]));
+    reinterpret_cast<float2 *>(c.pMUV)[q] = make_float2(to_float(mU), to_float(mV));
+    if (p.useAdaptiveEVP)
+        c.acf[q] = (float)(p.EVPcFac * f.recip_rA[o] / fmax(mC, 1e-4));
+    if (BASAL) c.bfac[q] = (float)basal_factor(p, f, o);
+    const bool south = is_neg(fc);
+    uint32_t fl = 0;
+    fl |= !is_zero(f.iceMask[o]) ? F_MC : 0;
+    fl |= !is_zero(f.maskInC[o]) ? F_INC : 0;
+    fl |= !is_zero(f.iceMaskU[o]) ? F_MU : 0;
+    fl |= !is_zero(f.maskInU[o]) ? F_INU : 0;
+    fl |= !is_zero(f.iceMaskV[o]) ? F_MV : 0;
+    fl |= !is_zero(f.maskInV[o]) ? F_INV : 0;
+    fl |= !is_zero(mU) ? F_LMU : 0;
+    fl |= !is_zero(mV) ? F_LMV : 0;
+    fl |= south ? F_SOUTH | F_SNEG : 0;
+    fl |= is_pos(fc) ? F_SPOS : 0;
+    c.flags16[q] = (uint16_t)fl;
+    if (j == 0)
+        reinterpret_cast<float4 *>(c.xm4)[i] = make_float4((float)f.recip_dxV[o], (float)f.recip_dxU[o],
+                                                           (float)f.dxU[o], (float)f.dxV[o]);
+    if (i == 0) {
+        c.rdyV_y[j] = (float)f.recip_dyV[o];
+        c.rdyU_y[j] = (float)f.recip_dyU[o];
+        c.dyV_y[j] = (float)f.dyV[o];
+        c.dyU_y[j] = (float)f.dyU[o];
+        c.qrA_y[j] = (float)(0.25 * f.recip_rA[o]);
+        c.rAz_y[j] = (float)f.rAz[o];
+        c.rrAu_y[j] = (float)f.recip_rAu[o];
+        c.rrAv_y[j] = (float)f.recip_rAv[o];
+    }
 }
 
 // ------------------------------------------------ shared-memory subcycle
@@ -219,10 +291,10 @@ int fast_prep(const Dims &d, const VerisParams &p, const Fields<double> &f, cons
     dim3 g2((d.NY + 31) / 32, (d.NX + 7) / 8);
     if (p.basalDragK2 != 0.0)
         fast_prep_kernel<T, true><<<g2, dim3(32, 8), 0, st>>>(p, f, d, lp, c, state0[0], state0[1], state0[2],
-                                                              state0[3], state0[4], 0);
+                                                              state0[3], state0[4]);
     else
         fast_prep_kernel<T, false><<<g2, dim3(32, 8), 0, st>>>(p, f, d, lp, c, state0[0], state0[1], state0[2],
-                                                               state0[3], state0[4], 0);
+                                                               state0[3], state0[4]);
     return launch_status();
 }
 
@@ -294,12 +366,25 @@ static int evp_fast(const VerisGrid *g, const VerisParams *p, const VerisFieldsF
     T *s0[5];
     for (int q = 0; q < 5; ++q) s0[q] = tape && !(rich && q >= 2) ? tslot(0, q) : state[0][q];
     dim3 g2((d.NY + 31) / 32, (d.NX + 7) / 8);
-    if (basal)
-        fast_prep_kernel<T, true><<<g2, dim3(32, 8), 0, st>>>(*p, f, d, lp, c, s0[0], s0[1], s0[2], s0[3], s0[4],
-                                                              paired ? 1 : 0);
-    else
-        fast_prep_kernel<T, false><<<g2, dim3(32, 8), 0, st>>>(*p, f, d, lp, c, s0[0], s0[1], s0[2], s0[3], s0[4],
-                                                               paired ? 1 : 0);
+    bool prepared = false;
+    if constexpr (sizeof(T) == 4) {
+        if (walker) {
+            Ctx<double> x;
+            x.f = f;
+            x.d = d;
+            x.p = *p;
+            float4 *quad = reinterpret_cast<float4 *>(s0[0]);
+            if (basal) walk_prep_kernel<true><<<g2, dim3(32, 8), 0, st>>>(x, lp, c, quad, s0[4]);
+            else walk_prep_kernel<false><<<g2, dim3(32, 8), 0, st>>>(x, lp, c, quad, s0[4]);
+            prepared = true;
+        }
+    }
+    if (!prepared) {
+        if (basal)
+            fast_prep_kernel<T, true><<<g2, dim3(32, 8), 0, st>>>(*p, f, d, lp, c, s0[0], s0[1], s0[2], s0[3], s0[4]);
+        else
+            fast_prep_kernel<T, false><<<g2, dim3(32, 8), 0, st>>>(*p, f, d, lp, c, s0[0], s0[1], s0[2], s0[3], s0[4]);
+    }
     int stt = launch_status();
     if (stt != VERIS_OK) return stt;
     const FastScalars<T> k = fast_scalars<T>(*p);
@@ -412,6 +497,18 @@ int veris_evp_fast_check(const VerisGrid *g, const VerisParams *p, const VerisFi
     if (cudaMemsetAsync(viol_device, 0, sizeof(int32_t), st) != cudaSuccess) return VERIS_ERR_LAUNCH;
     dim3 g2((d.NY + 31) / 32, (d.NX + 7) / 8);
     fast_check_kernel<<<g2, dim3(32, 8), 0, st>>>(*reinterpret_cast<const Fields<double> *>(vs), d, viol_device);
+    return launch_status();
+}
+
+int veris_evp_area_check(const VerisGrid *g, const VerisParams *p, const VerisFieldsF64 *vs, int32_t *viol_device,
+                         veris_stream_t s) {
+    Dims d;
+    VERIS_CHECK_GRID(g, d);
+    VERIS_REQUIRE(p && vs && viol_device, VERIS_ERR_ARG);
+    cudaStream_t st = (cudaStream_t)s;
+    if (cudaMemsetAsync(viol_device, 0, sizeof(int32_t), st) != cudaSuccess) return VERIS_ERR_LAUNCH;
+    dim3 g2((d.NY + 31) / 32, (d.NX + 7) / 8);
+    area_check_kernel<<<g2, dim3(32, 8), 0, st>>>(*reinterpret_cast<const Fields<double> *>(vs), d, viol_device);
     return launch_status();
 }
 

@@ -4,6 +4,7 @@
 #include <atomic>
 
 #include "evp_walk.cuh"
+#include "tile_units.cuh"
 
 namespace veris {
 namespace walk {
@@ -31,6 +32,7 @@ evp_walk_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<float> c, FastScalars
     const int w = blockIdx.x * WARPS + (threadIdx.x >> 5);
     if (w >= nwalks) return;   // whole warps only
     const int strip = w % nstrips, rb = w / nstrips;
+    chain_wait();
     // the single-domain walk takes the cell areas along j (the caller has
     // checked that the state's areas vary along j only: V_AREA2D clear)
     walk_strip<BASAL, TURN, Variant<V>::UNROLL, Variant<V>::PRE, ADAPT, (L != 0), (L == 1 || L == 3), true, false,
@@ -125,25 +127,23 @@ static int launch(const Dims &d, int64_t lp, const HaloFill &h, const FastConsts
                   const FastScalars<float> &k, const FastIO<float> &io, int H, cudaStream_t st) {
     const int nstrips = (d.NY + TW - 1) / TW, nblk = (d.NX + H - 1) / H;
     const int nwalks = nstrips * nblk;
-    evp_walk_kernel<B, R, V, A, L><<<(nwalks + WARPS - 1) / WARPS, WARPS * 32, 0, st>>>(d, lp, h, c, k, io,
-                                                                                   nstrips, nwalks, H);
-    return launch_status();
+    // chained without an early release: a walk's CTAs all run at once, and a
+    // successor's CTAs start as these end.  Per subcycle 90 x 40 12.0 -> 8.8 us,
+    // 360 x 180 10.4 -> 8.2, 1440 x 720 22.6 -> 20.2, 3600 x 1800 111.4 -> 108.9
+    // (released two, five or nine rows before the end 20.7, 21.0, 20.8 on 1440 x 720).
+    return launch_chained(evp_walk_kernel<B, R, V, A, L>, dim3((nwalks + WARPS - 1) / WARPS), dim3(WARPS * 32), 0,
+                          st, d, lp, h, c, k, io, nstrips, nwalks, H);
 }
 
 // walk length: the most rows per walk that still fits all walks in one wave
 // of resident warps (rows >= 8); ring overhead per walk is 4 rows
 template <bool B, bool R, int V, bool A, int L>
 static int auto_rows(const Dims &d) {
-    int dev = 0, sms = 0, per_sm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
-                                                  cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, evp_walk_kernel<B, R, V, A, L>, WARPS * 32, 0) !=
-            cudaSuccess || sms <= 0 || per_sm <= 0) {
-        cudaGetLastError();
-        return 16;
-    }
+    static std::atomic<int> resident[MAX_DEVICES];
+    const int slots = cta_slots(resident, evp_walk_kernel<B, R, V, A, L>, WARPS * 32, 0);
+    if (slots <= 0) return 16;
     const int strips = (d.NY + TW - 1) / TW;
-    const int blocks_per_wave = (sms * per_sm * WARPS) / strips;   // row blocks that fit next to each other
+    const int blocks_per_wave = (slots * WARPS) / strips;   // row blocks that fit next to each other
     if (blocks_per_wave < 1) return 16;
     int rows = (d.NX + blocks_per_wave - 1) / blocks_per_wave;
     return rows < 8 ? 8 : (rows > 4096 ? 4096 : rows);
@@ -261,6 +261,12 @@ int evp_walk_subcycles(bool adapt, bool paired, const Dims &d, const HaloFill &h
                        int rows, int variant, cudaStream_t st, bool paired_outs, int *status, float *const *rich) {
     const int64_t lp = internal_pitch(d.NY);
     if ((rows != 0 && (rows < 4 || rows > 4096)) || variant < 0 || variant >= walk::N_VARIANTS) return VERIS_ERR_ARG;
+    // Variant 3 (constants loaded a row early, four CTAs per SM) for grids whose
+    // state and constants, ~100 bytes a cell, leave the 126 MB L2: same values,
+    // 1800 x 900 30.3 us a subcycle against 32.6, 2400 x 1200 51.3 against 56.8,
+    // 3600 x 1800 108.9 against 120.4; below, 1600 x 800 25.1 against 24.8,
+    // 1440 x 720 20.3 against 20.2, 800 x 400 10.7 against 10.5.
+    if (variant == 0 && !rich && (int64_t)d.NX * d.NY >= (3 << 19)) variant = 3;
     if (rich && !(n == 1 && paired && paired_outs && !adapt && variant == 0)) return VERIS_ERR_ARG;
     int it0 = 0;
     if (paired && n >= 3 && status && walk::g_persistent.load(std::memory_order_relaxed)) {

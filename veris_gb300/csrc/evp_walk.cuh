@@ -57,7 +57,7 @@ struct Row {
 template <bool COH, class T>
 __device__ __forceinline__ T state_ld(const T *p) {
     if constexpr (COH) return __ldcg(p);
-    else return __ldg(p);
+    else return *p;
 }
 
 template <bool BASAL, bool ADAPT = false, bool PIN = false, bool A1D = false, bool COH = false>

@@ -151,6 +151,9 @@ __device__ __forceinline__ bool gt64(double a, double b) {   // a > b
     return order64(a) > order64(b) && !is_nan64(a) && !is_nan64(b) && !(is_zero(a) && is_zero(b));
 }
 
+__device__ __forceinline__ bool ne64(double a, double b) {   // a != b (true on NaN)
+    return (bits_of(a) != bits_of(b) && !(is_zero(a) && is_zero(b))) || is_nan64(a);
+}
 __device__ __forceinline__ bool ge64(double a, double b) {   // a >= b
     return !gt64(b, a) && !is_nan64(a) && !is_nan64(b);
 }
@@ -167,6 +170,18 @@ __device__ __forceinline__ float narrow(double x) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
     const unsigned e = min(max(hi & 0x7fffffffu, 0x38100000u), 0x47f00000u) - 0x38000000u;
     return __uint_as_float((hi & 0x80000000u) | (e << 3) | (lo >> 29));
+}
+
+// rounded to the nearest float, as a conversion, which takes a slot of the
+// float64 pipe; results outside the normal floats (but zeros) are converted
+__device__ __forceinline__ float to_float(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned mag = hi & 0x7fffffffu, sign = hi & 0x80000000u;
+    if (mag - 0x38100000u >= 0x0fe00000u && (mag | lo) != 0) return __double2float_rn(x);
+    unsigned f = ((mag - 0x38000000u) << 3) | (lo >> 29);
+    const unsigned rest = lo & 0x1fffffffu;
+    f += rest > 0x10000000u || (rest == 0x10000000u && (f & 1u)) ? 1u : 0u;
+    return __uint_as_float(sign | ((mag | lo) != 0 ? f : 0u));
 }
 
 // ------------------------------------------- exponential, logarithm, arctangent

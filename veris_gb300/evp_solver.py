@@ -99,7 +99,7 @@ def evp_solver_fast(state, precision="f32", form="tma", n_subcycles=None, return
     c = Call(state)
     if precision == "f32" and form == "walk":
         flag = torch.zeros(1, dtype=torch.int32, device=c.device)
-        check("evp_fast_check", c.lib.veris_evp_fast_check(*c.refs(), flag.data_ptr(), c.stream))
+        check("evp_area_check", c.lib.veris_evp_area_check(*c.refs(), flag.data_ptr(), c.stream))
         if int(flag.item()) & 128:
             raise ValueError("the register walk needs cell areas varying along j only (V_AREA2D set)")
     dt = torch.float32 if precision == "f32" else torch.float64
