@@ -23,9 +23,10 @@ namespace batch {
 
 // shapes 0-3: shared-memory tiles (rows x columns); 4-8: register walks of
 // 8, 16, 32, 64 or 128 rows over 28-column strips (one warp each; longer
-// walks recompute fewer ring rows, shorter ones balance better)
-constexpr int N_SHAPES = 9;
-constexpr int FIRST_WALK = 4;
+// walks recompute fewer ring rows, shorter ones balance better).  Table 9,
+// walks of 4 rows, is not a shape to ask for: see walk_shape().
+constexpr int N_SHAPES = 9, N_TABLES = 10;
+constexpr int FIRST_WALK = 4, SHORTEST_WALK = 9;
 template <int S>
 struct ShapeOf;
 template <>
@@ -38,8 +39,8 @@ template <>
 struct ShapeOf<3> { static constexpr int TI = 16, TJ = 16, MINB = 4; };
 
 inline void shape_dims(int s, int *ti, int *tj) {
-    static const int T[N_SHAPES][2] = {{32, 32}, {16, 32}, {32, 16}, {16, 16}, {8, 28}, {16, 28}, {32, 28},
-                                       {64, 28}, {128, 28}};
+    static const int T[N_TABLES][2] = {{32, 32}, {16, 32}, {32, 16}, {16, 16}, {8, 28}, {16, 28}, {32, 28},
+                                       {64, 28}, {128, 28}, {4, 28}};
     *ti = T[s][0];
     *tj = T[s][1];
 }
@@ -75,7 +76,7 @@ static int layout(int n, const VerisGrid *grids, size_t *queue, size_t *table, s
     *table = off;
     off += rup256((size_t)n * sizeof(Member));
     *tiles = off;
-    off += rup256((size_t)N_SHAPES * (n + 1) * sizeof(int));
+    off += rup256((size_t)N_TABLES * (n + 1) * sizeof(int));
     *members = off;
     size_t mo = 0;
     for (int m = 0; m < n; ++m) {
@@ -147,6 +148,7 @@ __global__ void __launch_bounds__(128, 4)
 evp_batch_walk_kernel(const Member *mem, const int *walk_start, int nmem, int nwalks, FastScalars<float> k, int buf,
                       unsigned *queue, unsigned base, int H) {
     const int lane = threadIdx.x & 31;
+    chain_wait();
     for (;;) {
         unsigned tk = 0;
         if (lane == 0) tk = atomicAdd(queue, 1u);
@@ -225,8 +227,8 @@ static int launch_s(bool basal, bool turn, const Member *mem, const int *ts, int
 template <bool B, bool R>
 static int launch_walk(const Member *mem, const int *ts, int nmem, int ntiles, const FastScalars<float> &k, int buf,
                        unsigned *queue, unsigned base, int blocks, int H, cudaStream_t st) {
-    evp_batch_walk_kernel<B, R><<<blocks, 128, 0, st>>>(mem, ts, nmem, ntiles, k, buf, queue, base, H);
-    return launch_status();
+    return launch_chained(evp_batch_walk_kernel<B, R>, dim3(blocks), dim3(128), 0, st, mem, ts, nmem, ntiles, k, buf,
+                          queue, base, H);
 }
 
 static int launch_walk_s(bool basal, bool turn, const Member *mem, const int *ts, int nmem, int ntiles,
@@ -237,6 +239,33 @@ static int launch_walk_s(bool basal, bool turn, const Member *mem, const int *ts
                     : launch_walk<true, false>(mem, ts, nmem, ntiles, k, buf, queue, base, blocks, H, st);
     return turn ? launch_walk<false, true>(mem, ts, nmem, ntiles, k, buf, queue, base, blocks, H, st)
                 : launch_walk<false, false>(mem, ts, nmem, ntiles, k, buf, queue, base, blocks, H, st);
+}
+
+// tiles or walks of all members in a shape; -1 for an invalid grid
+static int count_tiles(int n, const VerisGrid *grids, int shape) {
+    int ti, tj;
+    shape_dims(shape, &ti, &tj);
+    int acc = 0;
+    for (int m = 0; m < n; ++m) {
+        Dims d;
+        if (check_grid(&grids[m], &d) != VERIS_OK) return -1;
+        acc += ((d.NX + ti - 1) / ti) * ((d.NY + tj - 1) / tj);
+    }
+    return acc;
+}
+
+// The walk length that runs when walks of `shape` rows are asked for: the
+// longest at most that long whose walks occupy every warp slot of the launch
+// (the values do not depend on it).  With fewer, a subcycle lasts as long as
+// one walk whatever the members' size: 32-row walks took 47-52 us a subcycle
+// on 2 members (0.10 M cells), 4 (0.28 M) and 12 (0.90 M), 16-row walks 27, 29
+// and 35, 8-row walks 17, 19 and 35, 4-row walks 14 on 2; where they do, longer
+// walks repeat fewer ring rows: 60 members (3.7 M cells), 8, 16 and 32 rows
+// 124, 112 and 120 us.  (Chained launches take 2-3 us off each.)
+static int walk_shape(int n, const VerisGrid *grids, int shape, int warp_slots) {
+    while (shape != SHORTEST_WALK && count_tiles(n, grids, shape) < warp_slots)
+        shape = shape == FIRST_WALK ? SHORTEST_WALK : shape - 1;
+    return shape;
 }
 
 }  // namespace batch
@@ -259,13 +288,13 @@ int veris_batch_init(int32_t n, const VerisGrid *grids, const VerisParams *p, vo
     size_t q, t, ts, mb, total;
     Member *host = static_cast<Member *>(malloc((size_t)n * sizeof(Member)));
     size_t *moff = static_cast<size_t *>(malloc((size_t)n * sizeof(size_t)));
-    int *tiles = static_cast<int *>(malloc((size_t)N_SHAPES * (n + 1) * sizeof(int)));
+    int *tiles = static_cast<int *>(malloc((size_t)N_TABLES * (n + 1) * sizeof(int)));
     int st = (host && moff && tiles) ? layout(n, grids, &q, &t, &ts, &mb, &total, moff) : VERIS_ERR_ARG;
     if (st == VERIS_OK && wsb < total) st = VERIS_ERR_WORKSPACE;
     if (st == VERIS_OK) {
         char *base = static_cast<char *>(ws);
         for (int m = 0; m < n; ++m) host[m] = member_at(grids[m], *p, base + mb + moff[m]);
-        for (int s = 0; s < N_SHAPES; ++s) {
+        for (int s = 0; s < N_TABLES; ++s) {
             int ti, tj;
             shape_dims(s, &ti, &tj);
             int acc = 0;
@@ -276,7 +305,7 @@ int veris_batch_init(int32_t n, const VerisGrid *grids, const VerisParams *p, vo
             tiles[s * (n + 1) + n] = acc;
         }
         if (cudaMemcpy(base + t, host, (size_t)n * sizeof(Member), cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(base + ts, tiles, (size_t)N_SHAPES * (n + 1) * sizeof(int), cudaMemcpyHostToDevice) !=
+            cudaMemcpy(base + ts, tiles, (size_t)N_TABLES * (n + 1) * sizeof(int), cudaMemcpyHostToDevice) !=
                 cudaSuccess ||
             cudaMemset(base + q, 0, 256) != cudaSuccess)
             st = VERIS_ERR_LAUNCH;
@@ -289,15 +318,7 @@ int veris_batch_init(int32_t n, const VerisGrid *grids, const VerisParams *p, vo
 
 int veris_batch_tiles(int32_t n, const VerisGrid *grids, int32_t shape) {
     if (n < 1 || !grids || shape < 0 || shape >= N_SHAPES) return -1;
-    int ti, tj;
-    shape_dims(shape, &ti, &tj);
-    int acc = 0;
-    for (int m = 0; m < n; ++m) {
-        Dims d;
-        if (check_grid(&grids[m], &d) != VERIS_OK) return -1;
-        acc += ((d.NX + ti - 1) / ti) * ((d.NY + tj - 1) / tj);
-    }
-    return acc;
+    return count_tiles(n, grids, shape);
 }
 
 int veris_batch_prep_member_f32(int32_t n, const VerisGrid *grids, const VerisParams *p, void *ws, size_t wsb,
@@ -336,7 +357,12 @@ int veris_batch_evp_f32(int32_t n, const VerisGrid *grids, const VerisParams *p,
     int st = layout(n, grids, &q, &t, &ts, &mb, &total, nullptr);
     if (st != VERIS_OK) return st;
     VERIS_REQUIRE(wsb >= total, VERIS_ERR_WORKSPACE);
-    const int ntiles = veris_batch_tiles(n, grids, shape);
+    const int nsm = sm_count();
+    VERIS_REQUIRE(nsm > 0, VERIS_ERR_LAUNCH);
+    const bool walker = shape >= FIRST_WALK;
+    const int bps = blocks_per_sm > 0 ? blocks_per_sm : (walker ? 4 : 2);
+    if (walker) shape = walk_shape(n, grids, shape, nsm * bps * 4);
+    const int ntiles = count_tiles(n, grids, shape);
     VERIS_REQUIRE(ntiles > 0, VERIS_ERR_ARG);
     char *base = static_cast<char *>(ws);
     const Member *mem = reinterpret_cast<const Member *>(base + t);
@@ -354,10 +380,6 @@ int veris_batch_evp_f32(int32_t n, const VerisGrid *grids, const VerisParams *p,
         if ((st = launch_status()) != VERIS_OK) return st;
     }
     if (n_subcycles == 0) return VERIS_OK;
-    const int nsm = sm_count();
-    VERIS_REQUIRE(nsm > 0, VERIS_ERR_LAUNCH);
-    const bool walker = shape >= FIRST_WALK;
-    const int bps = blocks_per_sm > 0 ? blocks_per_sm : (walker ? 4 : 2);
     // tile kernels draw one ticket per CTA, the walk kernel one per warp;
     // every drawer ends on one ticket past the last
     const int blocks = walker ? min(nsm * bps, (ntiles + 3) / 4) : min(nsm * bps, ntiles);
