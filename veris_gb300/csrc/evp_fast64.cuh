@@ -18,15 +18,13 @@
 //   update's coefficient), one multiplication fewer per use; the drag
 //   coefficient is the square root of the product the drag floor's test
 //   forms;
-// * divisions and square roots start from the hardware's approximate
-//   reciprocal and reciprocal square root (rcp/rsqrt.approx.ftz.f64) and
-//   add the first terms of the series of the exact correction: with
-//   e = 1 - b*r0, 1/b = r0/(1 - e) = r0*(1 + e + e^2 + ...); with
-//   s0 = x*y and r = 1 - s0*y, sqrt(x) = s0*(1 - r)^(-1/2) = s0*(1 + r/2 +
-//   3r^2/8 + ...) (the Newton-Raphson correction taken to second order,
-//   P. Markstein, IBM J. Res. Dev. 34 (1990) 111).  Four and five float64
-//   instructions, no slow path; a warp whose operands leave a safe exponent
-//   range uses IEEE division or square root instead;
+// * divisions and square roots run in integer and float32 instructions
+//   (f64math.cuh), of which the schedulers could issue ten times as many as
+//   they do beside the float64 pipe: with the hardware's seeds and float64
+//   series (four and five float64 operations each, 22 of 90 per cell)
+//   1440 x 720 took 191 us a subcycle and 360 x 180 20.1, now 166 and 17.0; a
+//   warp whose operands leave a safe exponent range uses IEEE division or
+//   square root instead;
 // * warps whose cells all have zero ice strength skip the viscosity's
 //   square root and division (zeta = 0, which the formula gives), warps on
 //   land skip the velocity division;

@@ -1,28 +1,16 @@
-// Float64 division, reciprocal and square root from the hardware's
-// approximate reciprocal and reciprocal square root, for kernels bound by
-// GB300's float64 pipe (2 lanes per SM and cycle).
-//
-// rcp.approx.ftz.f64 and rsqrt.approx.ftz.f64 give about 20 correct bits;
-// the first terms of the series of the exact correction finish the job:
-// with e = 1 - b*r0, 1/b = r0/(1 - e) = r0*(1 + e + e^2 + ...); with
-// s0 = x*y and r = 1 - s0*y, sqrt(x) = s0*(1 - r)^(-1/2) = s0*(1 + r/2 +
-// 3r^2/8 + ...) and 1/sqrt(x) = y*(1 + r/2 + 3r^2/8 + ...) (Newton-Raphson
-// taken to second order in series form, P. Markstein, IBM J. Res. Dev. 34
-// (1990) 111).  Three to five float64 instructions, no slow path; a warp
-// whose operands leave a safe exponent range takes IEEE division or square
-// root instead.  Zero tests run on the integer pipe.
+// Float64 arithmetic off the float64 pipe, for kernels that it bounds: GB300
+// has 2 float64 lanes per SM and cycle, 1/64 of its float32 rate.  Division and
+// square root in integer and float32 instructions, comparisons and conversions
+// on the integer pipe, table-driven exponential, logarithm and arctangent; the
+// reciprocal square root from the hardware's seed and the series of the exact
+// correction.  No slow paths inside: a lane or warp whose operands leave a safe
+// exponent range takes IEEE division or square root instead.
 #pragma once
 #include <cuda_runtime.h>
 
 #include "f64tables.cuh"
 
 namespace veris {
-
-__device__ __forceinline__ double rcp_seed(double b) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
-    return r;
-}
 
 __device__ __forceinline__ double rsqrt_seed(double x) {
     double r;
@@ -31,7 +19,7 @@ __device__ __forceinline__ double rsqrt_seed(double x) {
 }
 
 // positive, normal, and at least 2^64 away from both ends of the exponent
-// range (so neither the seed nor its square flushes or overflows)
+// range (so neither a seed nor its square flushes or overflows)
 __device__ __forceinline__ bool seed_range(double b) {
     const int hi = __double2hiint(b);
     return hi >= (64 << 20) && hi < (1984 << 20);
@@ -47,27 +35,87 @@ __device__ __forceinline__ unsigned long long bits_of(double x) {
 
 __device__ __forceinline__ bool is_zero(double x) { return (bits_of(x) << 1) == 0; }
 
-// a / b for b in seed_range: r0 ~ 1/b, e = 1 - b*r0, 1/b = r0*(1 + e + e^2 + O(e^3))
-__device__ __forceinline__ double div_series(double a, double b) {
-    const double r0 = rcp_seed(b);
-    const double e = fma(-b, r0, 1.0);
-    return a * fma(r0, fma(e, e, e), r0);
+// Division and square root without the float64 pipe: it takes a warp's
+// instruction every 64 cycles per scheduler, in which the scheduler issues as
+// many integer and float32 instructions.  With the significands as 53-bit
+// integers, a double-float quotient (root) is good to 2^-45, so an integer Q
+// within 2^9 of the scaled result; the remainder, exact modulo 2^64 by three
+// 32-bit products (its size is below 2^63), divided in float32 gives the
+// integer correction.  The result is within 0.51 units in the last place.
+// About fifty instructions each, against four and five on the float64 pipe
+// (reciprocal and reciprocal square root seeds and their series).
+
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// the significand of a normal value: its leading 24 bits as a float in [1, 2),
+// the other 29 as a float in units of 2^-52
+__device__ __forceinline__ float lead24(unsigned hi, unsigned lo) {
+    return __uint_as_float((__funnelshift_l(lo, hi, 3) & 0x007fffffu) | 0x3f800000u);
+}
+__device__ __forceinline__ float rest29(unsigned lo) { return (float)(int)(lo & 0x1fffffffu); }
+
+// a / b, b in seed_range, a 0 or of such a magnitude, the quotient's exponent
+// in the normal range (div_range)
+__device__ __forceinline__ bool div_range(double a, double b) {
+    const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = __double2hiint(b) >> 20;
+    return eb >= 64 && eb < 1984 && (is_zero(a) || ((unsigned)(ea - 64) < 1920u && (unsigned)(ea - eb + 1020) < 2040u));
+}
+__device__ __forceinline__ double div_int(double a, double b) {
+    const unsigned ah = (unsigned)__double2hiint(a), al = (unsigned)__double2loint(a);
+    const unsigned bh = (unsigned)__double2hiint(b), bl = (unsigned)__double2loint(b);
+    const float fa = lead24(ah, al), fb = lead24(bh, bl);
+    float r = rcp_approx(fb);
+    r = fmaf(r, fmaf(-fb, r, 1.f), r);
+    const float q0 = __fmul_rn(fa, r);
+    const float rm = fmaf(fmaf(-q0, rest29(bl), rest29(al)), 0x1p-52f, fmaf(-q0, fb, fa));
+    const unsigned long long ma = ((unsigned long long)(ah & 0xfffffu) << 32) | al,
+                             mb = ((unsigned long long)(bh & 0xfffffu) << 32) | bl;
+    const int lt = ma < mb ? 1 : 0;   // quotient below 1
+    const int i0 = __float2int_rn(q0 * 0x1p24f), i1 = __float2int_rn(rm * (r * 0x1p52f));
+    const unsigned long long Q = (unsigned long long)(((long long)i0 << 28) + i1) << lt;
+    const unsigned Ql = (unsigned)Q, Qh = (unsigned)(Q >> 32);
+    const unsigned P = __umulhi(Ql, bl) + Ql * ((bh & 0xfffffu) | 0x100000u) + Qh * bl;
+    const int rem = (int)((al << (20 + lt)) - P);   // high word of (ma << (52 + lt)) - Q mb
+    const int d = __float2int_rn((float)rem * (r * 0x1p-20f));
+    const int e = (int)((ah >> 20) & 0x7ffu) - (int)(bh >> 20) + 1022 - lt;
+    const unsigned long long z = Q + (long long)d + ((unsigned long long)(unsigned)e << 52);
+    const double q = __longlong_as_double((long long)(z | ((unsigned long long)(ah & 0x80000000u) << 32)));
+    return (((ah << 1) | al) == 0) ? a : q;
 }
 
-// sqrt(x) for x in seed_range: y ~ x^(-1/2), s0 = x*y, r = 1 - s0*y,
-// sqrt(x) = s0*(1 - r)^(-1/2) = s0*(1 + r/2 + 3r^2/8 + O(r^3))
-__device__ __forceinline__ double sqrt_series(double x) {
-    const double y = rsqrt_seed(x);
-    const double s0 = x * y;
-    const double r = fma(-s0, y, 1.0);
-    return fma(s0, r * fma(0.375, r, 0.5), s0);
+// sqrt(x) for x in seed_range
+__device__ __forceinline__ double sqrt_int(double x) {
+    const unsigned xh = (unsigned)__double2hiint(x), xl = (unsigned)__double2loint(x);
+    const int odd = ((xh >> 20) & 1) ^ 1;   // the unbiased exponent's parity
+    const float fx = odd ? 2.f * lead24(xh, xl) : lead24(xh, xl);
+    float y = rsqrt_approx(fx);
+    float s0 = __fmul_rn(fx, y);
+    y = fmaf(0.5f * y, fmaf(-s0, y, 1.f), y);
+    s0 = __fmul_rn(fx, y);
+    const float rm = fmaf(rest29(xl), odd ? 0x1p-51f : 0x1p-52f, fmaf(-s0, s0, fx));
+    const int i0 = __float2int_rn(s0 * 0x1p24f), i1 = __float2int_rn(rm * (y * 0x1p51f));
+    const unsigned long long S = (unsigned long long)(((long long)i0 << 28) + i1);
+    const unsigned Sl = (unsigned)S, Sh = (unsigned)(S >> 32);
+    const unsigned P = __umulhi(Sl, Sl) + Sl * (Sh << 1);
+    const int rem = (int)((xl << (20 + odd)) - P);   // high word of (m << (52 + odd)) - S^2
+    const int d = __float2int_rn((float)rem * (y * 0x1p-21f));
+    const int e = (((int)(xh >> 20) - 1023) >> 1) + 1022;
+    return __longlong_as_double((long long)(S + (long long)d + ((unsigned long long)(unsigned)e << 52)));
 }
 
 // a / b on the lanes of `m` (all of which call it); IEEE division for the
-// whole warp when any b leaves the seed range (zero, denormal, negative,
-// huge, NaN)
+// whole warp when any operand or quotient leaves the safe range (b zero,
+// denormal, negative, huge or NaN; a denormal, huge or NaN)
 __device__ __forceinline__ double div64(double a, double b, unsigned m) {
-    if (__all_sync(m, seed_range(b))) return div_series(a, b);
+    if (__all_sync(m, div_range(a, b))) return div_int(a, b);
     return a / b;
 }
 
@@ -75,7 +123,7 @@ __device__ __forceinline__ double div64(double a, double b, unsigned m) {
 __device__ __forceinline__ double sqrt64(double x, unsigned m) {
     const bool z = is_zero(x);
     if (__all_sync(m, z || seed_range(x))) {
-        const double s = sqrt_series(z ? 1.0 : x);
+        const double s = sqrt_int(z ? 1.0 : x);
         return z ? 0.0 : s;
     }
     return sqrt(x);
@@ -88,14 +136,12 @@ __device__ __forceinline__ bool gt_nonneg(double x, double y) {
 }
 
 // 1/b for b in seed_range
-__device__ __forceinline__ double rcp_series(double b) {
-    const double r0 = rcp_seed(b);
-    const double e = fma(-b, r0, 1.0);
-    return fma(r0, fma(e, e, e), r0);
-}
+__device__ __forceinline__ double rcp_int(double b) { return div_int(1.0, b); }
 
-// 1/sqrt(x) for x in seed_range: y ~ x^(-1/2), r = 1 - x*y^2,
-// x^(-1/2) = y*(1 - r)^(-1/2) = y*(1 + r/2 + 3r^2/8 + O(r^3))
+// 1/sqrt(x) for x in seed_range: y ~ x^(-1/2) (20 bits), r = 1 - x*y^2,
+// x^(-1/2) = y*(1 - r)^(-1/2) = y*(1 + r/2 + 3r^2/8 + O(r^3)) (Newton-Raphson
+// taken to second order in series form, P. Markstein, IBM J. Res. Dev. 34
+// (1990) 111)
 __device__ __forceinline__ double rsqrt_series(double x) {
     const double y = rsqrt_seed(x);
     const double r = fma(-(x * y), y, 1.0);
@@ -105,7 +151,7 @@ __device__ __forceinline__ double rsqrt_series(double x) {
 // 1/b on the lanes of `m`; IEEE division for the whole warp when any b
 // leaves the seed range
 __device__ __forceinline__ double rcp64(double b, unsigned m) {
-    if (__all_sync(m, seed_range(b))) return rcp_series(b);
+    if (__all_sync(m, seed_range(b))) return rcp_int(b);
     return 1.0 / b;
 }
 
@@ -119,12 +165,12 @@ __device__ __forceinline__ double rsqrt64(double x, unsigned m) {
 // known (data-dependent branches): the series where the operand is in the
 // seed range, IEEE otherwise (a warp whose lanes disagree runs both).
 __device__ __forceinline__ double div_lane(double a, double b) {
-    return seed_range(b) ? div_series(a, b) : a / b;
+    return div_range(a, b) ? div_int(a, b) : a / b;
 }
-__device__ __forceinline__ double rcp_lane(double b) { return seed_range(b) ? rcp_series(b) : 1.0 / b; }
+__device__ __forceinline__ double rcp_lane(double b) { return seed_range(b) ? rcp_int(b) : 1.0 / b; }
 __device__ __forceinline__ double sqrt_lane(double x) {
     if (is_zero(x)) return x;
-    return seed_range(x) ? sqrt_series(x) : sqrt(x);
+    return seed_range(x) ? sqrt_int(x) : sqrt(x);
 }
 __device__ __forceinline__ double rsqrt_lane(double x) { return seed_range(x) ? rsqrt_series(x) : 1.0 / sqrt(x); }
 
@@ -241,7 +287,7 @@ __device__ __forceinline__ double atan_table(double x) {
     if ((unsigned)(hi - 0x3ff00000) > (unsigned)(0x400ccccc - 0x3ff00000)) return ::atan(x);
     const int k = (int)fmaf(narrow(x), 64.f, -63.5f);   // 64 (x - 1), rounded
     const double c = widen(fmaf((float)k, 0.015625f, 1.f));
-    const double d = div_series(x - c, fma(x, c, 1.0));
+    const double d = div_int(x - c, fma(x, c, 1.0));
     const double d2 = d * d;
     const float f = narrow(d2);
     const double q = widen(f * fmaf(f, -1.f / 7.f, 0.2f)) - 1.0 / 3.0;

@@ -29,9 +29,9 @@
 // last three, seaice_global_4deg.py:761).
 //
 // Both routines are bound by GB300's float64 pipe in float64 (2 lanes per SM
-// and cycle): their divisions, reciprocals and square roots take the
-// series-refined hardware approximations of f64math.cuh (per lane, IEEE
-// where an operand leaves the safe range).  In float32 the bulk formula is
+// and cycle): their divisions, reciprocals and square roots take the integer
+// and float32 forms of f64math.cuh (per lane, IEEE where an operand leaves the
+// safe range).  In float32 the bulk formula is
 // bound by instruction issue: its divisions, logarithms, exponential and the
 // square roots of the psi functions use the hardware approximations
 // (__fdividef, __logf, __expf, rsqrtf: a few units in
@@ -238,13 +238,14 @@ __global__ void __launch_bounds__(256) bulkf_kernel(BulkArgs<T> a) {
 // bulkf_kernel with the table-driven logarithm, arctangent and exponential
 // (7, 11 and 8 float64 operations), square roots and reciprocals without
 // range checks where the scheme bounds the operand, comparisons on the
-// integer pipe, and the iteration's constants folded: 49 float64 operations
-// per unstable iteration, 8 per stable one.
+// integer pipe, and the iteration's constants folded: 32 float64 operations
+// per unstable iteration, two per stable one.
 //   psi_m = 2 ln((1 + x)/2) + 2 ln((1 + x^2)/2) - 2 atan x + pi/2,
 //   psi_h = 2 ln((1 + x^2)/2), x = (1 - 16 huol)^(1/4);
 //   Dm, Dh = 1 + g (aln - psi) = c0 - g psi
 // 1444 x 724 points, half of them unstable: 1.50 ms with CUDA's log, atan and
-// exp (170 operations per unstable iteration); here 0.67 ms.
+// exp (170 operations per unstable iteration); 0.67 ms with reciprocal and
+// square root series on the float64 pipe; here 0.48 ms.
 __global__ void __launch_bounds__(256) bulkf64_kernel(BulkArgs<double> a, double c0) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < a.n;
          k += (int64_t)gridDim.x * blockDim.x) {
@@ -265,9 +266,9 @@ __global__ void __launch_bounds__(256) bulkf64_kernel(BulkArgs<double> a, double
             if ((unsigned)(__double2hiint(h) & 0x7fffffff) >= 0x40240000u && !is_nan64(h))
                 h = __hiloint2double((__double2hiint(h) & 0x80000000) | 0x40240000, 0);
             if (is_neg(h)) {
-                const double s = sqrt_series(fma(-16.0, h, 1.0));
+                const double s = sqrt_int(fma(-16.0, h, 1.0));
                 const double xsq = __double2hiint(s) < 0x3ff00000 ? 1.0 : s;
-                const double x = sqrt_series(xsq);
+                const double x = sqrt_int(xsq);
                 const double l2 = 2.0 * log_table(fma(0.5, xsq, 0.5));
                 const double lx = log_table(fma(0.5, x, 0.5));
                 const double psim = fma(-2.0, atan_table(x), fma(2.0, lx, l2)) + 1.57079632679489661923;
