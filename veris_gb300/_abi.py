@@ -6,7 +6,9 @@ settings into the ``VerisParams`` struct.  The library is required: there is
 no CPU fallback, and a missing or unloadable library raises ``VerisError``.
 """
 import ctypes
+import operator
 import os
+import struct
 
 import numpy as np
 
@@ -70,6 +72,26 @@ class VerisFields(ctypes.Structure):
 BULK_PARAMS = ("zvir", "cpdair", "karman", "latvap", "ocean_emissivity", "gamma_blk", "grav")
 DERIVED_PARAMS = ("EVPcFac", "sinWin", "cosWin", "sinWatOcn", "cosWatOcn",
                   "s4t_cc0", "s4t_cc1", "s4t_cc2", "s4t_d1", "s4t_d1i", "pad_")
+# the settings that are packed as they are, read in one call, and their places in the struct
+_PLAIN_DOUBLES = [n for n in PARAM_DOUBLES if n not in DERIVED_PARAMS]
+_PLAIN_INTS = [n for n in PARAM_INTS if n not in DERIVED_PARAMS]
+_read_doubles = operator.attrgetter(*_PLAIN_DOUBLES)
+_read_ints = operator.attrgetter(*_PLAIN_INTS)
+_DOUBLE_AT = [PARAM_DOUBLES.index(n) for n in _PLAIN_DOUBLES]
+_DERIVED_AT = {n: PARAM_DOUBLES.index(n) for n in DERIVED_PARAMS if n != "pad_"}
+_PACK = struct.Struct("=%dd%di" % (len(PARAM_DOUBLES), len(PARAM_INTS)))
+assert _PLAIN_INTS == PARAM_INTS[:-1] and _PACK.size == ctypes.sizeof(VerisParams)
+# saturation constants of veris/solve4temp.py:14-27
+_CC0 = 10 ** 12.537
+_CC1 = float(_CC0 * 2663.5 * 0.622 * 100000 * np.log(10))
+_CC2 = float(_CC0 * (1 - 0.622))
+
+
+def _sin_cos(degrees):
+    if degrees == 0:
+        return 0.0, 1.0
+    r = np.deg2rad(degrees)
+    return float(np.sin(r)), float(np.cos(r))
 
 
 def params_from_settings(sett):
@@ -80,35 +102,26 @@ def params_from_settings(sett):
     veris/evp_solver.py:264-268, veris/solve4temp.py:14-27), so both sides
     start from identically rounded constants.
     """
-    from .settings import SETTINGS
-    p = VerisParams()
-    for n in PARAM_DOUBLES:
-        if n in DERIVED_PARAMS:
-            continue
-        if n in BULK_PARAMS and not hasattr(sett, n):
-            # host-model constants of the bulk formulae; settings saved before
-            # they were carried here hold the defaults
-            setattr(p, n, float(SETTINGS[n][0]))
-            continue
-        setattr(p, n, float(getattr(sett, n)))
-    for n in PARAM_INTS:
-        if n in DERIVED_PARAMS:
-            continue
-        setattr(p, n, int(getattr(sett, n)))
-    p.sinWin = float(np.sin(np.deg2rad(sett.airTurnAngle)))
-    p.cosWin = float(np.cos(np.deg2rad(sett.airTurnAngle)))
-    p.sinWatOcn = float(np.sin(np.deg2rad(sett.waterTurnAngle)))
-    p.cosWatOcn = float(np.cos(np.deg2rad(sett.waterTurnAngle)))
-    p.EVPcFac = float(sett.deltatDyn * 4 * (np.pi * sett.aEvpCoeff) ** 2) if sett.useAdaptiveEVP else 0.0
-    aa1, aa2, bb1, pa = 2663.5, 12.537, 0.622, 100000
-    cc0 = 10 ** aa2
-    p.s4t_cc0 = float(cc0)
-    p.s4t_cc1 = float(cc0 * aa1 * bb1 * pa * np.log(10))
-    p.s4t_cc2 = float(cc0 * (1 - bb1))
-    p.s4t_d1 = float(sett.dalton * sett.cpAir * sett.rhoAir)
-    p.s4t_d1i = float(sett.dalton * sett.lhSublim * sett.rhoAir)
-    p.pad_ = 0
-    return p
+    try:
+        plain = _read_doubles(sett)
+    except AttributeError:
+        # host-model constants of the bulk formulae; settings saved before
+        # they were carried here hold the defaults
+        from .settings import SETTINGS
+        plain = [SETTINGS[n][0] if n in BULK_PARAMS and not hasattr(sett, n) else getattr(sett, n)
+                 for n in _PLAIN_DOUBLES]
+    v = [0.0] * len(PARAM_DOUBLES)
+    for k, x in zip(_DOUBLE_AT, plain):
+        v[k] = float(x)
+    d = _DERIVED_AT
+    v[d["sinWin"]], v[d["cosWin"]] = _sin_cos(sett.airTurnAngle)
+    v[d["sinWatOcn"]], v[d["cosWatOcn"]] = _sin_cos(sett.waterTurnAngle)
+    if sett.useAdaptiveEVP:
+        v[d["EVPcFac"]] = float(sett.deltatDyn * 4 * (np.pi * sett.aEvpCoeff) ** 2)
+    v[d["s4t_cc0"]], v[d["s4t_cc1"]], v[d["s4t_cc2"]] = _CC0, _CC1, _CC2
+    v[d["s4t_d1"]] = float(sett.dalton * sett.cpAir * sett.rhoAir)
+    v[d["s4t_d1i"]] = float(sett.dalton * sett.lhSublim * sett.rhoAir)
+    return VerisParams.from_buffer_copy(_PACK.pack(*v, *map(int, _read_ints(sett)), 0))
 
 
 _P = ctypes.c_void_p

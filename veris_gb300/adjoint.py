@@ -13,7 +13,7 @@ import ctypes
 
 import torch
 
-from ._abi import VerisFields, check
+from ._abi import VerisFields, check, load
 from .state import Call
 
 EVP_STATE = ("uIce", "vIce", "sigma1", "sigma2", "sigma12")
@@ -108,13 +108,13 @@ def _pointwise4(name, fn, state, lam_out):
 def cleanup_adjoint(state, lam_out):
     """Adjoint of clean_up_advection followed by ridging (veris/clean_up.py:5-47)
     for (hIceMean, hSnowMean, Area, TSurf) at ``state``."""
-    return _pointwise4("cleanup_adjoint", Call(state).lib.veris_cleanup_adjoint_f64, state, lam_out)
+    return _pointwise4("cleanup_adjoint", load().veris_cleanup_adjoint_f64, state, lam_out)
 
 
 def growth_adjoint(state, lam_out):
     """Adjoint of Growth (veris/growth.py:8-397) for (hIceMean, hSnowMean, Area,
     TSurf) at ``state``, whose forcing fields must be the ones Growth read."""
-    return _pointwise4("growth_adjoint", Call(state).lib.veris_growth_adjoint_f64, state, lam_out)
+    return _pointwise4("growth_adjoint", load().veris_growth_adjoint_f64, state, lam_out)
 
 
 def prep_adjoint(state, lam_prep):

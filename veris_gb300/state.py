@@ -5,6 +5,9 @@ Mirrors the host model's state interface that the plugin's kernels read
 the variables held as CUDA tensors (PyTorch owns the memory).  Every
 variable is a 2-D ``(nx + 4, ny + 4)`` tensor, y contiguous.
 """
+import ctypes
+import functools
+import struct
 from types import SimpleNamespace
 
 import numpy as np
@@ -52,8 +55,15 @@ def require_device(t, name, dtype, shape):
     return t if t.is_contiguous() else t.contiguous()
 
 
+_FIELD_PACK = struct.Struct("=%dQ" % len(ABI_ORDER))
+
+
 class Call:
-    """Grid, params and field table of one C-ABI call, with keep-alive refs."""
+    """Grid, params and field table of one C-ABI call, with keep-alive refs.
+
+    Every variable present is checked on every call; the table is packed at
+    once (one struct member at a time, and the settings likewise, took most
+    of a small routine's time on the host)."""
 
     def __init__(self, state, dtype=torch.float64, variables=None):
         v = state.variables if variables is None else variables
@@ -61,22 +71,27 @@ class Call:
         ref = v.iceMask
         if ref.dim() != 2:
             raise ValueError("state variables must be 2-D")
-        self.shape = tuple(ref.shape)
+        self.shape = shape = tuple(ref.shape)
         self.dtype = dtype
         self.device = ref.device
-        NX, NY = self.shape
+        NX, NY = shape
         olx, oly = int(sett.olx), int(sett.oly)
         self.grid = _abi.VerisGrid(NX - 2 * olx, NY - 2 * oly, olx, oly, NY)
         self.params = _abi.params_from_settings(sett)
-        self.fields = _abi.VerisFields()
-        self.keep = []
+        self.keep = keep = []
+        get = vars(v).get if type(v) in (Variables, SimpleNamespace) else functools.partial(_get, v)
+        ptrs = []
         for n in ABI_ORDER:
-            t = getattr(v, n, None)
+            t = get(n)
             if t is None:
+                ptrs.append(0)
                 continue
-            t = require_device(t, n, dtype, self.shape)
-            self.keep.append(t)
-            setattr(self.fields, n, t.data_ptr())
+            if not (type(t) is torch.Tensor and t.dtype is dtype and t.is_cuda and t.shape == shape and
+                    t.is_contiguous()):
+                t = require_device(t, n, dtype, shape)
+            keep.append(t)
+            ptrs.append(t.data_ptr())
+        self.fields = _abi.VerisFields.from_buffer_copy(_FIELD_PACK.pack(*ptrs))
         self.stream = torch.cuda.current_stream(self.device).cuda_stream
         self.lib = _abi.load()
 
@@ -95,9 +110,8 @@ class Call:
         return ws.data_ptr(), ws.numel()
 
     def refs(self):
-        return (ctypes_ref(self.grid), ctypes_ref(self.params), ctypes_ref(self.fields))
+        return (ctypes.byref(self.grid), ctypes.byref(self.params), ctypes.byref(self.fields))
 
 
-def ctypes_ref(x):
-    import ctypes
-    return ctypes.byref(x)
+def _get(v, name):
+    return getattr(v, name, None)
