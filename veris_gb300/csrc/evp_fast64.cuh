@@ -93,7 +93,7 @@ inline F64Scalars f64_scalars(const FastScalars<double> &k, double sideU0 = 0.0)
 }
 
 // ------------------------------------------------------------------ tile
-constexpr int F64_THREADS = 256;
+constexpr int F64_THREADS = 256, F64_WIDE = 768;
 
 // TI output rows x 32 columns per CTA; 16-, 24- and 32-row tiles fit 4, 3
 // and 2 CTAs per SM (smaller tiles: more resident warps, more ring work)
@@ -119,7 +119,7 @@ static_assert(3 * (Smem64<16>::bytes(true, true, true) + 1024) <= 228 * 1024, "t
 // The plain tile in a CTA of the folded form's launch: the settings and field
 // table come through shared memory behind the tile's arrays.  Not inlined:
 // the folded form keeps its registers.
-template <int TI, bool ADAPT, bool SLIP, bool BASAL>
+template <int TI, bool ADAPT, bool SLIP, bool BASAL, int NT>
 __device__ __noinline__ void plain_fallback(const Ctx<double> *ctx, HaloFill h, FastIO<double> io, int i0, int ti,
                                             int j0) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -127,16 +127,16 @@ __device__ __noinline__ void plain_fallback(const Ctx<double> *ctx, HaloFill h, 
     static_assert(at + sizeof(Ctx<double>) <= Smem64<TI>::bytes(BASAL, ADAPT, SLIP), "the plain tile's shared memory");
     Ctx<double> *c = reinterpret_cast<Ctx<double> *>(smem_raw + at);
     static_assert(sizeof(Ctx<double>) % sizeof(int) == 0, "copied by words");
-    for (int q = threadIdx.x; q < (int)(sizeof(Ctx<double>) / sizeof(int)); q += F64_THREADS)
+    for (int q = threadIdx.x; q < (int)(sizeof(Ctx<double>) / sizeof(int)); q += NT)
         reinterpret_cast<int *>(c)[q] = reinterpret_cast<const int *>(ctx)[q];
     __syncthreads();
     const EvpIO<double> p{io.u, io.v, io.s1, io.s2, io.s12, io.uo, io.vo, io.s1o, io.s2o, io.s12o,
                           c->f.uIce, c->f.vIce, io.aCo};
-    plain_tile<double, TI, ADAPT, SLIP, BASAL>(smem_raw, *c, h, p, i0, ti, j0);
+    plain_tile<double, TI, ADAPT, SLIP, BASAL, NT>(smem_raw, *c, h, p, i0, ti, j0);
 }
 
-template <int TI, bool BASAL, bool TURN, bool TAPE, bool ADAPT = false, bool SLIP = false, bool AUTO = false>
-__global__ void __launch_bounds__(F64_THREADS, (ADAPT || SLIP) ? 3 : f64_min_blocks(TI))
+template <int TI, bool BASAL, bool TURN, bool TAPE, bool ADAPT, bool SLIP, bool AUTO, int NT>
+__global__ void __launch_bounds__(NT, NT > F64_THREADS ? 1 : ((ADAPT || SLIP) ? 3 : f64_min_blocks(TI)))
 evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars k, FastIO<double> io,
                TileUnits w, F64Auto a) {
     using S = Smem64<TI>;
@@ -174,12 +174,12 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
     chain_wait();
     if (AUTO) {
         if (*a.viol) {   // the same for every CTA and subcycle
-            plain_fallback<TI, ADAPT, SLIP, BASAL>(a.ctx, h, io, i0, ti, j0);
+            plain_fallback<TI, ADAPT, SLIP, BASAL, NT>(a.ctx, h, io, i0, ti, j0);
             return;
         }
     }
     // ---- stage u, v and the flags of the tile plus a 2-cell ring
-    for (int idx = tid; idx < nS; idx += F64_THREADS) {
+    for (int idx = tid; idx < nS; idx += NT) {
         const int li = idx / S::WS - 2, lj = idx % S::WS - 2;
         const int64_t o = (int64_t)d.wxt(i0 + li) * lp + d.wyt(j0 + lj);
         sU[idx] = io.u[o];
@@ -189,7 +189,7 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
     __syncthreads();
 
     // ---- A: e12 at Z points [-1, TI+1] x [-1, TJ+1] (veris/dynamics_routines.py:160-175)
-    for (int base = 0; base < nZ; base += F64_THREADS) {
+    for (int base = 0; base < nZ; base += NT) {
         const int idx = base + tid;
         const unsigned m = __ballot_sync(ALL, idx < nZ);
         if (idx >= nZ) continue;
@@ -221,7 +221,7 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
 
     // ---- B: viscosities at C [-1, TI] x [-1, TJ] (veris/dynamics_routines.py:220-268);
     //      stresses, drag and Coriolis terms on [-1, TI) x [-1, TJ) (veris/evp_solver.py:80-145)
-    for (int base = 0; base < nB; base += F64_THREADS) {
+    for (int base = 0; base < nB; base += NT) {
         const int idx = base + tid;
         const unsigned m = __ballot_sync(ALL, idx < nB);
         if (idx >= nB) continue;
@@ -320,7 +320,7 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
 
     // ---- C: sigma12 at Z [0, TI] x [0, TJ] (veris/evp_solver.py:101-103 with
     //      veris/averaging.py:4-19); sZq is dead: it takes sigma12
-    for (int idx = tid; idx < nC; idx += F64_THREADS) {
+    for (int idx = tid; idx < nC; idx += NT) {
         const int li = idx / S::WC, lj = idx % S::WC;
         const int gi = d.wxt(i0 + li), gj = d.wyt(j0 + lj);
         const uint32_t n = (sF[IS(li, lj)] & F_MC) + (sF[IS(li - 1, lj)] & F_MC) + (sF[IS(li, lj - 1)] & F_MC) +
@@ -348,7 +348,7 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
     chain_release();
 
     // ---- D: u, v at the tile's U and V points (veris/evp_solver.py:105-187)
-    for (int base = 0; base < ti * S::TJ; base += F64_THREADS) {
+    for (int base = 0; base < ti * S::TJ; base += NT) {
         const int idx = base + tid;
         const int li = idx / S::TJ, lj = idx % S::TJ;
         const int gi = i0 + li, gj = j0 + lj;
@@ -445,19 +445,35 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
 #undef IZZ
 }
 
-template <int TI, bool B, bool R, bool TP, bool AD = false, bool SL = false, bool AUTO = false>
-static int launch64(const Dims &d, int64_t lp, const HaloFill &h, const FastConsts<double> &c, const F64Scalars &k,
-                    const FastIO<double> &io, cudaStream_t st, const F64Auto &a = F64Auto{}) {
+template <int TI, bool B, bool R, bool TP, bool AD, bool SL, bool AUTO, int NT>
+static int launch64_tile(const Dims &d, int64_t lp, const HaloFill &h, const FastConsts<double> &c, const F64Scalars &k,
+                    const FastIO<double> &io, cudaStream_t st, const F64Auto &a) {
     using S = Smem64<TI>;
-    auto kern = evp_f64_kernel<TI, B, R, TP, AD, SL, AUTO>;
+    auto kern = evp_f64_kernel<TI, B, R, TP, AD, SL, AUTO, NT>;
     const size_t sm = S::bytes(B, AD, SL);
     static std::atomic<bool> configured[MAX_DEVICES];
     if (!smem_configured(configured, kern, (int)sm)) return VERIS_ERR_LAUNCH;
     static std::atomic<int> resident[MAX_DEVICES];
-    const int slots = cta_slots(resident, kern, F64_THREADS, sm);
+    const int slots = cta_slots(resident, kern, NT, sm);
     if (slots <= 0) return VERIS_ERR_LAUNCH;
+    if (NT == F64_WIDE && (int64_t)((d.NY + S::TJ - 1) / S::TJ) * ((d.NX + TI - 1) / TI) > slots)
+        return VERIS_ERR_UNSUPPORTED;
     const TileUnits w = tile_units(d, TI, slots);
-    return launch_chained(kern, dim3(w.count), dim3(F64_THREADS), sm, st, d, lp, h, c, k, io, w, a);
+    return launch_chained(kern, dim3(w.count), dim3(NT), sm, st, d, lp, h, c, k, io, w, a);
+}
+
+// Grids that one 16-row piece per SM covers take one CTA of 768 threads per SM:
+// as many warps as three of 256, on pieces three times as tall, whose rings are
+// a smaller part of the work.  Per subcycle, three CTAs / one: 128 x 64
+// 10.4 / 8.6 us, 180 x 90 11.0 / 9.0, 240 x 121 12.3 / 10.7, 360 x 180 17.1 / 15.8;
+// with taller pieces the three win, 443 x 221 23.5 / 25.0, 600 x 300 35.0 / 45.6.
+// (384 threads x 2: 9.5, 9.5, 11.5, 16.9; 512 x 1: 8.4, 8.7, 10.5, 18.9.)
+template <int TI, bool B, bool R, bool TP, bool AD = false, bool SL = false, bool AUTO = false>
+static int launch64(const Dims &d, int64_t lp, const HaloFill &h, const FastConsts<double> &c, const F64Scalars &k,
+                    const FastIO<double> &io, cudaStream_t st, const F64Auto &a = F64Auto{}) {
+    const int stt = launch64_tile<16, B, R, TP, AD, SL, AUTO, F64_WIDE>(d, lp, h, c, k, io, st, a);
+    if (stt != VERIS_ERR_UNSUPPORTED) return stt;
+    return launch64_tile<TI, B, R, TP, AD, SL, AUTO, F64_THREADS>(d, lp, h, c, k, io, st, a);
 }
 
 }  // namespace veris

@@ -50,8 +50,8 @@ struct PlainSmem {
 };
 
 // rows [i0, i0 + ti) (ti <= TI) and columns [j0, j0 + 32) of one subcycle, by
-// the EVP_THREADS threads of the CTA
-template <class T, int TI, bool ADAPT, bool SIDE, bool BASAL>
+// the NT threads of the CTA
+template <class T, int TI, bool ADAPT, bool SIDE, bool BASAL, int NT = EVP_THREADS>
 __device__ __forceinline__ void plain_tile(unsigned char *smem_raw, const Ctx<T> &c, const HaloFill &h,
                                            const EvpIO<T> &io, int i0, int ti, int j0) {
     using S = PlainSmem<T, TI, ADAPT, SIDE, BASAL>;
@@ -82,7 +82,7 @@ __device__ __forceinline__ void plain_tile(unsigned char *smem_raw, const Ctx<T>
 #define ZZ(li, lj) (li) * S::WC + (lj)
 
     // ---- stage A: e12 at Z points
-    for (int idx = tid; idx < nZ; idx += EVP_THREADS) {
+    for (int idx = tid; idx < nZ; idx += NT) {
         const int li = idx / S::WZ - 1, lj = idx % S::WZ - 1;
         const int gi = i0 + li, gj = j0 + lj;
         if (gi >= d.NX + 2 || gj >= d.NY + 2) continue;   // feeds no stored point; keeps the wrap within one period
@@ -95,7 +95,7 @@ __device__ __forceinline__ void plain_tile(unsigned char *smem_raw, const Ctx<T>
     // ---- stage B: viscosities and the C-point stress update
     const T alpha = T(c.p.evpAlpha);
     const T rdenom = T(1.0 / c.p.evpAlpha);
-    for (int idx = tid; idx < nB; idx += EVP_THREADS) {
+    for (int idx = tid; idx < nB; idx += NT) {
         const int li = idx / S::WB - 1, lj = idx % S::WB - 1;
         const int gi = i0 + li, gj = j0 + lj;
         if (gi >= d.NX + 2 || gj >= d.NY + 2) continue;   // feeds no stored point; keeps the wrap within one period
@@ -140,7 +140,7 @@ __device__ __forceinline__ void plain_tile(unsigned char *smem_raw, const Ctx<T>
     __syncthreads();
 
     // ---- stage C: sigma12 at Z points
-    for (int idx = tid; idx < nC; idx += EVP_THREADS) {
+    for (int idx = tid; idx < nC; idx += NT) {
         const int li = idx / S::WC, lj = idx % S::WC;
         const int gi = i0 + li, gj = j0 + lj;
         if (gi >= d.NX + 2 || gj >= d.NY + 2) continue;   // feeds no stored point; keeps the wrap within one period
@@ -165,7 +165,7 @@ __device__ __forceinline__ void plain_tile(unsigned char *smem_raw, const Ctx<T>
     const T rdt = T(c.p.recip_deltatDyn);
     const T cosW = T(c.p.cosWat), sinW = T(c.p.sinWat);
     const T beta = T(c.p.evpBeta);
-    for (int idx = tid; idx < ti * TJ; idx += EVP_THREADS) {
+    for (int idx = tid; idx < ti * TJ; idx += NT) {
         const int li = idx / TJ, lj = idx % TJ;
         const int gi = i0 + li, gj = j0 + lj;
         if (gi >= d.NX || gj >= d.NY) continue;
