@@ -804,22 +804,20 @@ static int evp_adjoint(const VerisGrid *g, const VerisParams *p, const VerisFiel
                 const LamG<T> ll = lam_of(ss, lb);
                 const int lb_next = first ? 0 : lb ^ 1;
                 bool done = false;
-                if constexpr (sizeof(T) == 4) {
-                    // float32 without turning angle: P4 of each subcycle fused with P1 of the one
-                    // before it in the segment
-                    if (!turn && f32_form != 3) {
-                        const bool head = ss == s1 - 1;
-                        if (ss > s0) {
-                            const TapeG<T> tp = tape_of(ss - 1);
-                            const LamG<T> lpv = lam_of(ss - 1, lb_next);
-                            stt = adjoint_gather_chain<T>(d, lp, h, pl.c, k, p->rhoSea, tt, ll, pl.a, pl.scr, basal,
-                                                          head, &tp, &lpv, st);
-                        } else {
-                            stt = adjoint_gather_chain<T>(d, lp, h, pl.c, k, p->rhoSea, tt, ll, pl.a, pl.scr, basal,
-                                                          head, nullptr, nullptr, st);
-                        }
-                        done = true;
+                // without turning angle: P4 of each subcycle fused with P1 of the one before it in
+                // the segment
+                if (!turn && (sizeof(T) == 8 || f32_form != 3)) {
+                    const bool head = ss == s1 - 1;
+                    if (ss > s0) {
+                        const TapeG<T> tp = tape_of(ss - 1);
+                        const LamG<T> lpv = lam_of(ss - 1, lb_next);
+                        stt = adjoint_gather_chain<T>(d, lp, h, pl.c, k, p->rhoSea, tt, ll, pl.a, pl.scr, basal,
+                                                      head, &tp, &lpv, st);
+                    } else {
+                        stt = adjoint_gather_chain<T>(d, lp, h, pl.c, k, p->rhoSea, tt, ll, pl.a, pl.scr, basal,
+                                                      head, nullptr, nullptr, st);
                     }
+                    done = true;
                 }
                 if (!done)
                     stt = adjoint_gather_subcycle<T>(d, lp, h, pl.c, k, p->rhoSea, tt, ll, pl.a, pl.scr, basal, turn,

@@ -20,20 +20,30 @@
 //       Coriolis, ocean and basal drag adjoints;
 //   P4  U and V points: the gathered velocity and ocean-velocity adjoints.
 //
-// In float32 without a turning angle, P4 of each subcycle and P1 of the
-// subcycle before it run as one pass (uv_link_kernel): what P4 gathers at a
-// point is what that P1 reads there.  On grids of more CTAs than the GPU
-// holds at once, the float32 P3 and the fused pass are bounded to 32
-// registers (eight CTAs per SM): latency-bound, they gain more from the
-// resident warps than they lose to spills.
+// Without a turning angle, P4 of each subcycle and P1 of the subcycle
+// before it run as one pass (uv_link_kernel): what P4 gathers at a point is
+// what that P1 reads there.  On grids of more CTAs than the GPU holds at
+// once, the float32 P3 and the fused pass are bounded to 32 registers:
+// latency-bound, they gain more from the resident warps than they lose to
+// spills.
+//
+// The passes are chained (common.cuh): the next one is resident when its
+// predecessor ends.  In float64 each computes what depends on the tape and
+// the constants alone (reciprocals, strain rates, e12, the drag's branch)
+// before it waits: no pass of the sweep writes those, and what wrote them is
+// complete, since P1 at the head of a sweep and every pass after an
+// unchained kernel start ordinarily.  The wait then covers only the gathers.
+// The sweep on 360 x 180 with its forward, 30 subcycles float64: 1866 us with
+// four passes started one after another, 1580 so; 90 x 40, 60 subcycles 1980
+// and 1577.
 //
 // Every point is computed once, nothing is recomputed on rings and nothing
 // is accumulated with atomics (each input adjoint is written by the pass
 // that owns its position).  In float64 the forward's Delta, zeta and drag
 // coefficient come from the tape the float64 forward writes (evp_fast.cu),
 // so the adjoint takes no square root of the forward's; its reciprocals and
-// the basal drag's reciprocal square root use the series-refined hardware
-// approximations of f64math.cuh, masks are selects and zero tests run on the
+// the basal drag's reciprocal square root run in integer and float32
+// instructions (f64math.cuh), masks are selects and zero tests run on the
 // integer pipe.  A float32 tape (the register walk's) holds the walk's own
 // Delta, zeta and drag coefficient beside its state; a float32 segment
 // recomputed from a checkpoint does not, and two first passes recompute e12,
@@ -55,7 +65,7 @@ namespace adj {
 namespace {
 
 constexpr unsigned ALL = 0xffffffffu;
-constexpr int BX = 32, BY = 8;   // 32 points along j (contiguous) x 8 rows per 256-thread block
+constexpr int BX = 32, BY = 4;   // 32 points along j (contiguous) x 4 rows per 128-thread block
 
 // the step's scalars, products folded once on the host
 template <class T>
@@ -69,6 +79,7 @@ struct KT {
     T kXN, kXS;                // (rhoSea drag)^2 / 4: 2 d cDrag/dX = kX / cDrag
     double wN, wS;             // rhoSea / (rhoSea drag): d cDrag / d drag = cDrag * w
     T U02;                     // basal U0^2
+    bool early;                // the passes release their successor at their start
 };
 
 template <class T>
@@ -134,8 +145,8 @@ __device__ __forceinline__ bool z_wet(uint32_t f0, uint32_t fw, uint32_t fs, uin
 template <class T>
 __device__ __forceinline__ T sel(bool b, T x) { return b ? x : T(0); }
 
-// the arithmetic of each precision: float64 on the series-refined hardware
-// approximations (f64math.cuh), float32 IEEE-rounded
+// the arithmetic of each precision: float64 in integer and float32
+// instructions (f64math.cuh), float32 IEEE-rounded
 template <class T>
 struct Fp;
 template <>
@@ -334,24 +345,81 @@ __device__ __forceinline__ void own_adjoints(const Dims &d, const HaloFill &h, c
 // luo, lvo: ocean-velocity adjoint shares of the subcycle after it (its P4
 // run in the same kernel), added to a.uOc, a.vOc before this subcycle's
 // (the order of the separate passes); MERGE: there are such shares
-template <class T, bool BASAL, bool TURN, bool MERGE>
-__device__ __forceinline__ void p1_point(const Dims &d, int64_t lp, const FastConsts<T> &c, const TapeG<T> &t,
-                                         const LamG<T> &l, const Adj<T> &a, const KT<T> &k, const Scr<T> &s,
-                                         unsigned m, int i, int j, T LU, T LV, T luo, T lvo) {
+// what P1 needs of a U or V point that no pass of the sweep writes: the
+// subcycle's tape and constants
+template <class T>
+struct P1Half {
+    T hA, K, S, o, x, xn, r;   // cos/2 A, the drag sum times it, the sum, ocean and ice velocity, its result, 1/den
+    T cb;                      // sum of the two basal coefficients
+    bool any, guard;           // a wet point in this warp; the denominator was 0
+};
+template <class T>
+struct P1Pre {
+    P1Half<T> U, V;
+    T cd0, cdw, cds;
+    uint32_t f0;
+};
+
+template <class T, bool BASAL>
+__device__ __forceinline__ P1Pre<T> p1_prepare(const Dims &d, int64_t lp, const FastConsts<T> &c, const TapeG<T> &t,
+                                               const KT<T> &k, const Scr<T> &s, unsigned m, int i, int j) {
     const Fold<T> F{c, k};
     const int iw = wxp(d, i - 1), js = wyp(d, j - 1);
     const int64_t o = (int64_t)i * lp + j, ow = (int64_t)iw * lp + j, os = (int64_t)i * lp + js;
-    const uint32_t f0 = c.flags[o];
-    const T cd0 = t.cd[o], cdw = t.cd[ow], cds = t.cd[os];
+    P1Pre<T> q;
+    q.f0 = c.flags[o];
+    q.cd0 = t.cd[o];
+    q.cdw = t.cd[ow];
+    q.cds = t.cd[os];
     T cb0 = T(0), cbw = T(0), cbs = T(0);
     if (BASAL) {
         cb0 = s.cb[o];
         cbw = s.cb[ow];
         cbs = s.cb[os];
     }
+    q.U.any = __any_sync(m, q.f0 & F_MU);
+    if (q.U.any) {   // hAW = cos/2 AW, mUb1 = mU (beta+1)/dt
+        q.U.hA = F.hAW(o);
+        q.U.o = c.uOc[o];
+        q.U.x = t.U(o);
+        q.U.xn = t.UN(o);
+        q.U.S = q.cd0 + q.cdw;
+        q.U.K = q.U.hA * q.U.S;
+        q.U.cb = cb0 + cbw;
+        T den = F.mUb1(o) + q.U.K;
+        if (BASAL) den = fma(T(0.5) * c.AW[o], q.U.cb, den);
+        q.U.guard = Fp<T>::zero(den);
+        q.U.r = Fp<T>::rcp(q.U.guard ? T(1) : den, m);
+    }
+    q.V.any = __any_sync(m, q.f0 & F_MV);
+    if (q.V.any) {
+        q.V.hA = F.hAS(o);
+        q.V.o = c.vOc[o];
+        q.V.x = t.V(o);
+        q.V.xn = t.VN(o);
+        q.V.S = q.cd0 + q.cds;
+        q.V.K = q.V.hA * q.V.S;
+        q.V.cb = cb0 + cbs;
+        T den = F.mVb1(o) + q.V.K;
+        if (BASAL) den = fma(T(0.5) * c.AS[o], q.V.cb, den);
+        q.V.guard = Fp<T>::zero(den);
+        q.V.r = Fp<T>::rcp(q.V.guard ? T(1) : den, m);
+    }
+    return q;
+}
+
+template <class T, bool BASAL, bool TURN, bool MERGE>
+__device__ __forceinline__ void p1_point(const Dims &d, int64_t lp, const FastConsts<T> &c, const TapeG<T> &t,
+                                         const LamG<T> &l, const Adj<T> &a, const KT<T> &k, const Scr<T> &s,
+                                         const P1Pre<T> &q, int i, int j, T LU, T LV, T luo, T lvo) {
+    const Fold<T> F{c, k};
+    const int iw = wxp(d, i - 1), js = wyp(d, j - 1);
+    const int64_t o = (int64_t)i * lp + j, ow = (int64_t)iw * lp + j, os = (int64_t)i * lp + js;
+    const uint32_t f0 = q.f0;
+    const T cd0 = q.cd0, cdw = q.cdw, cds = q.cds;
     T sg = T(0);
     if (TURN) sg = (f0 & F_SPOS) ? T(1) : ((f0 & F_SNEG) ? T(-1) : T(0));
-    if (!__any_sync(m, f0 & F_MU)) {   // a warp of dry U points: no momentum adjoint, nothing to add
+    if (!q.U.any) {   // a warp of dry U points: no momentum adjoint, nothing to add
         if (MERGE) a.uOc[o] += luo;
         l.ou[o] = T(0);
         s.gU[o] = T(0);
@@ -359,15 +427,10 @@ __device__ __forceinline__ void p1_point(const Dims &d, int64_t lp, const FastCo
         s.wU0[o] = T(0);
         if (TURN) s.wU1[o] = s.q0U[o] = s.qwU[o] = T(0);
         if (BASAL) s.bU[o] = T(0);
-    } else {   // U point (hAW = cos/2 AW, mUb = mU beta/dt, mUb1 = mU (beta+1)/dt)
-        const T hA = F.hAW(o), uo = c.uOc[o], u0 = t.U(o);
-        const T S = cd0 + cdw, kU = hA * S;
-        T den = F.mUb1(o) + kU;
-        if (BASAL) den = fma(T(0.5) * c.AW[o], cb0 + cbw, den);
-        const bool guard = Fp<T>::zero(den);
-        const T r = Fp<T>::rcp(guard ? T(1) : den, m);
-        const T g = sel<T>(f0 & F_MU, LU * r);
-        const T lden = guard ? T(0) : -t.UN(o) * g;
+    } else {   // U point (mUb = mU beta/dt)
+        const T hA = q.U.hA, uo = q.U.o, u0 = q.U.x, S = q.U.S, kU = q.U.K;
+        const T g = sel<T>(f0 & F_MU, LU * q.U.r);
+        const T lden = q.U.guard ? T(0) : -q.U.xn * g;
         const T Y = fma(uo, g, lden);   // d/dkU
         const T W = hA * Y;
         l.ou[o] = F.mUb(o) * g;
@@ -375,7 +438,7 @@ __device__ __forceinline__ void p1_point(const Dims &d, int64_t lp, const FastCo
         a.cU[o] += g;
         T lAW = fma(k.hc * S, Y, a.AW[o]);
         if (BASAL) {
-            lAW = fma(T(0.5) * (cb0 + cbw), lden, lAW);
+            lAW = fma(T(0.5) * q.U.cb, lden, lAW);
             s.bU[o] = T(0.5) * c.AW[o] * lden;
         }
         a.uOc[o] = fma(kU, g, MERGE ? a.uOc[o] + luo : a.uOc[o]);
@@ -399,7 +462,7 @@ __device__ __forceinline__ void p1_point(const Dims &d, int64_t lp, const FastCo
         }
         a.AW[o] = lAW;
     }
-    if (!__any_sync(m, f0 & F_MV)) {
+    if (!q.V.any) {
         if (MERGE) a.vOc[o] += lvo;
         l.ov[o] = T(0);
         s.gV[o] = T(0);
@@ -408,14 +471,9 @@ __device__ __forceinline__ void p1_point(const Dims &d, int64_t lp, const FastCo
         if (TURN) s.wV1[o] = s.q0V[o] = s.qsV[o] = T(0);
         if (BASAL) s.bV[o] = T(0);
     } else {   // V point
-        const T hA = F.hAS(o), vo = c.vOc[o], v0 = t.V(o);
-        const T S = cd0 + cds, kV = hA * S;
-        T den = F.mVb1(o) + kV;
-        if (BASAL) den = fma(T(0.5) * c.AS[o], cb0 + cbs, den);
-        const bool guard = Fp<T>::zero(den);
-        const T r = Fp<T>::rcp(guard ? T(1) : den, m);
-        const T g = sel<T>(f0 & F_MV, LV * r);
-        const T lden = guard ? T(0) : -t.VN(o) * g;
+        const T hA = q.V.hA, vo = q.V.o, v0 = q.V.x, S = q.V.S, kV = q.V.K;
+        const T g = sel<T>(f0 & F_MV, LV * q.V.r);
+        const T lden = q.V.guard ? T(0) : -q.V.xn * g;
         const T Y = fma(vo, g, lden);
         const T W = hA * Y;
         l.ov[o] = F.mVb(o) * g;
@@ -423,7 +481,7 @@ __device__ __forceinline__ void p1_point(const Dims &d, int64_t lp, const FastCo
         a.cV[o] += g;
         T lAS = fma(k.hc * S, Y, a.AS[o]);
         if (BASAL) {
-            lAS = fma(T(0.5) * (cb0 + cbs), lden, lAS);
+            lAS = fma(T(0.5) * q.V.cb, lden, lAS);
             s.bV[o] = T(0.5) * c.AS[o] * lden;
         }
         a.vOc[o] = fma(kV, g, MERGE ? a.vOc[o] + lvo : a.vOc[o]);
@@ -455,10 +513,13 @@ __global__ void __launch_bounds__(BX * BY) uv_reverse_kernel(Dims d, int64_t lp,
     const int j = blockIdx.x * BX + threadIdx.x, i = blockIdx.y * BY + threadIdx.y;
     const bool act = i < d.NX && j < d.NY;
     const unsigned m = __ballot_sync(ALL, act);
+    chain_wait();
+    if (k.early) chain_release();
     if (!act) return;
     T LU, LV;
     own_adjoints(d, h, l, i, j, LU, LV);
-    p1_point<T, BASAL, TURN, false>(d, lp, c, t, l, a, k, s, m, i, j, LU, LV, T(0), T(0));
+    const P1Pre<T> q = p1_prepare<T, BASAL>(d, lp, c, t, k, s, m, i, j);
+    p1_point<T, BASAL, TURN, false>(d, lp, c, t, l, a, k, s, q, i, j, LU, LV, T(0), T(0));
 }
 
 // ------------------------------------------------------------------ P2
@@ -470,23 +531,35 @@ __global__ void __launch_bounds__(BX * BY) z_reverse_kernel(Dims d, int64_t lp, 
     const int j = blockIdx.x * BX + threadIdx.x, i = blockIdx.y * BY + threadIdx.y;
     const bool act = i < d.NX && j < d.NY;
     const unsigned m = __ballot_sync(ALL, act);
-    if (!act) return;
     const Fold<T> F{c, k};
     const int iw = wxp(d, i - 1), js = wyp(d, j - 1);
     const int64_t o = (int64_t)i * lp + j, ow = (int64_t)iw * lp + j, os = (int64_t)i * lp + js,
                   ows = (int64_t)iw * lp + js;
+    T e = T(0), zs = T(0), e2 = T(0), nh = T(0);
+    if (sizeof(T) == 4) {
+        chain_wait();
+        if (k.early) chain_release();
+    }
+    if (act) {   // of the tape and the constants
+        const uint32_t f0 = c.flags[o], fw = c.flags[ow], fs = c.flags[os], fws = c.flags[ows];
+        const uint32_t n = (f0 & F_MC) + (fw & F_MC) + (fs & F_MC) + (fws & F_MC);
+        nh = n == 4 ? k.nh4 : (n == 3 ? k.nh3 : (n == 2 ? k.nh2 : (n == 1 ? k.nh1 : T(0))));
+        e = e12_ready ? s.e12[o] : e12_at(F, t, m, i, j, o, ow, os, f0, fw, fs, fws);
+        zs = (t.zeta[o] + t.zeta[ow]) + (t.zeta[os] + t.zeta[ows]);
+        e2 = c.rAz[o] * e;
+    }
+    if (sizeof(T) == 8) {
+        chain_wait();
+        if (k.early) chain_release();
+    }
+    if (!act) return;
     // sigma12' at Z(i, j) enters sdx of U(i, j) (-) and U(i, j-1) (+), sdy of V(i, j) (-) and V(i-1, j) (+)
     const T L = fma(c.dxV_x[i], s.rU[os] - s.rU[o], fma(c.dyU_y[j], s.rV[ow] - s.rV[o], l.ls12[(int64_t)i * l.ldl + j]));
     l.os12[o] = k.am1 * L;
-    const uint32_t f0 = c.flags[o], fw = c.flags[ow], fs = c.flags[os], fws = c.flags[ows];
-    const uint32_t n = (f0 & F_MC) + (fw & F_MC) + (fs & F_MC) + (fws & F_MC);
-    const T nh = n == 4 ? k.nh4 : (n == 3 ? k.nh3 : (n == 2 ? k.nh2 : (n == 1 ? k.nh1 : T(0))));
-    const T e = e12_ready ? s.e12[o] : e12_at(F, t, m, i, j, o, ow, os, f0, fw, fs, fws);
-    const T zs = (t.zeta[o] + t.zeta[ow]) + (t.zeta[os] + t.zeta[ows]);
     const T cz = nh * L;
     s.tZ[o] = cz * e;
     s.le12[o] = cz * zs;
-    s.e2[o] = c.rAz[o] * e;
+    s.e2[o] = e2;
 }
 
 // ------------------------------------------------------------------ P3
@@ -502,13 +575,85 @@ __device__ __forceinline__ void c_reverse_body(const Dims &d, int64_t lp, const 
     const bool act = i < d.NX && j < d.NY;
     const unsigned m = __ballot_sync(ALL, act);
     T dragN = T(0), dragS = T(0);   // float32: this warp's water-drag terms
+    const Fold<T> F{c, k};
+    const int ie = wxp(d, i + 1), jn = wyp(d, j + 1);
+    const int64_t o = (int64_t)i * lp + j, oe = (int64_t)ie * lp + j, on = (int64_t)i * lp + jn,
+                  oen = (int64_t)ie * lp + jn;
+    // of the tape and the constants: strain rates, the reciprocals, the drag's branch (taken
+    // exactly as the forward takes it)
+    uint32_t f0 = 0;
+    T u0 = T(0), ue = T(0), v0 = T(0), vn = T(0), rdx = T(0), rdy = T(0), ep = T(0), em = T(0), del = T(0),
+      zeta = T(0), rz = T(0), rdel = T(0), A = T(0), B = T(0), cd = T(0), rc = T(0), rs = T(0);
+    bool live = false, dz = false, fast = false;
+    uint32_t fe = 0, fn = 0;
+    auto strain = [&]() {
+        const bool inC = f0 & F_INC;
+        u0 = t.U(o);
+        ue = t.U(oe);
+        v0 = t.V(o);
+        vn = t.V(on);
+        rdx = c.rdxU_x[i];
+        rdy = c.rdyV_y[j];
+        const T e11 = inC ? (ue - u0) * rdx : T(0);
+        const T e22 = inC ? (vn - v0) * rdy : T(0);
+        ep = e11 + e22;
+        em = e11 - e22;
+        del = t.del[o];
+        zeta = t.zeta[o];
+    };
+    auto recip_zeta = [&]() { rz = Fp<T>::rcp(del + k.dmin, m); };
+    auto recip_delta = [&]() {
+        live = __any_sync(m, !Fp<T>::zero(zeta));
+        if (live) {
+            dz = Fp<T>::zero(del);
+            rdel = Fp<T>::rcp(dz ? T(1) : del, m);
+        }
+    };
+    auto drag = [&]() {
+        // ocean drag: cd = 0.5 rhoSea drag sqrt(X), X = (du + du_e)^2 + (dv + dv_n)^2, above its floor
+        const T du0 = (f0 & F_INU) ? u0 - c.uOc[o] : T(0);
+        const T du1 = (fe & F_INU) ? ue - c.uOc[oe] : T(0);
+        const T dv0 = (f0 & F_INV) ? v0 - c.vOc[o] : T(0);
+        const T dv1 = (fn & F_INV) ? vn - c.vOc[on] : T(0);
+        A = du0 + du1;
+        B = dv0 + dv1;
+        const T X = fma(B, B, A * A);
+        fast = (f0 & F_MC) && Fp<T>::gt(((f0 & F_SOUTH) ? k.dcq2S : k.dcq2N) * X, k.cmin2);
+        if (__any_sync(m, fast)) {
+            cd = t.cd[o];
+            rc = Fp<T>::rcp(fast ? cd : T(1), m);
+        }
+    };
+    auto basal = [&]() {
+        // cb = bfac / sqrt(0.25 (a^2 + b^2 + c^2 + e^2) + U0^2), a = inU u, b = inU_e u_e, c = inV v, e = inV_n v_n
+        const T a_ = sel<T>(f0 & F_INU, u0), b_ = sel<T>(fe & F_INU, ue);
+        const T c_ = sel<T>(f0 & F_INV, v0), e_ = sel<T>(fn & F_INV, vn);
+        const T qb = T(0.25) * (a_ * a_ + b_ * b_ + c_ * c_ + e_ * e_) + k.U02;
+        rs = Fp<T>::rsqrt(qb, m);
+    };
+    constexpr bool EARLY = sizeof(T) == 8;
+    if (!EARLY) {
+        chain_wait();
+        if (k.early) chain_release();
+    }
     if (act) {
-        const Fold<T> F{c, k};
-        const int ie = wxp(d, i + 1), jn = wyp(d, j + 1);
-        const int64_t o = (int64_t)i * lp + j, oe = (int64_t)ie * lp + j, on = (int64_t)i * lp + jn,
-                      oen = (int64_t)ie * lp + jn;
-        const uint32_t f0 = c.flags[o], fe = c.flags[oe], fn = c.flags[on];
-        const bool mC = f0 & F_MC, inC = f0 & F_INC;
+        f0 = c.flags[o];
+        fe = c.flags[oe];
+        fn = c.flags[on];
+        if (EARLY) {
+            strain();
+            recip_zeta();
+            recip_delta();
+            drag();
+            if (BASAL) basal();
+        }
+    }
+    if (EARLY) {
+        chain_wait();
+        if (k.early) chain_release();
+    }
+    if (act) {
+        const bool mC = f0 & F_MC, inC = f0 & F_INC, south = f0 & F_SOUTH;
         // shares gathered from U(i, j), U(i+1, j), V(i, j), V(i, j+1)
         const T sU = s.gU[o] + s.gU[oe], sV = s.gV[o] + s.gV[on];
         const T lcd = (s.wU0[o] + (TURN ? s.wU1[oe] : s.wU0[oe])) + (s.wV0[o] + (TURN ? s.wV1[on] : s.wV0[on]));
@@ -523,26 +668,19 @@ __device__ __forceinline__ void c_reverse_body(const Dims &d, int64_t lp, const 
         // sigma1' = mC ((alpha-1)/alpha sigma1 + zeta (2 ep - kp Delta)/alpha),
         // sigma2' = mC ((alpha-1)/alpha sigma2 + zeta em/(2 alpha)): h1 = 2 d/dsigma1'/alpha, h2 = d/dsigma2'/(2 alpha)
         const T h1 = sel<T>(mC, k.ra2 * L1), h2 = sel<T>(mC, k.rah * L2);
-        // strain rates (recomputed from the tape's velocities)
-        const T u0 = t.U(o), ue = t.U(oe), v0 = t.V(o), vn = t.V(on);
-        const T rdx = c.rdxU_x[i], rdy = c.rdyV_y[j];
-        const T e11 = inC ? (ue - u0) * rdx : T(0);
-        const T e22 = inC ? (vn - v0) * rdy : T(0);
-        const T ep = e11 + e22, em = e11 - e22;
-        const T del = t.del[o], zeta = t.zeta[o];
+        if (!EARLY) strain();
         const T tz = (s.tZ[o] + s.tZ[oe]) + (s.tZ[on] + s.tZ[oen]);
         const T lz = fma(fma(-k.hkp, del, ep), h1, fma(em, h2, tz));
         // zeta = Ph/(Delta + Delta_min)
-        const T rz = Fp<T>::rcp(del + k.dmin, m);
+        if (!EARLY) recip_zeta();
         a.Ph[o] = fma(lz, rz, a.Ph[o]);
         // where the ice strength is 0, zeta = 0 and nothing flows back through Delta
         T q = T(0), le11 = T(0), le22 = T(0);
-        if (__any_sync(m, !Fp<T>::zero(zeta))) {
+        if (!EARLY) recip_delta();
+        if (live) {
             T lep = zeta * h1, lem = zeta * h2;
             const T ldel = fma(-zeta * rz, lz, -k.hkp * lep);
             // Delta = sqrt(ep^2 + rsq em^2 + (recip_rA/e^2) sum rAz e12^2); 0 at Delta = 0.  q = 2 dL/dDelta^2
-            const bool dz = Fp<T>::zero(del);
-            const T rdel = Fp<T>::rcp(dz ? T(1) : del, m);
             q = dz ? T(0) : ldel * rdel;
             lep = fma(ep, q, lep);
             lem = fma(k.rsq * em, q, lem);
@@ -559,36 +697,19 @@ __device__ __forceinline__ void c_reverse_body(const Dims &d, int64_t lp, const 
         s.uB[o] = fu + le11;
         s.vA[o] = fv - le22;
         s.vB[o] = fv + le22;
-        // ocean drag: cd = 0.5 rhoSea drag sqrt(X), X = (du + du_e)^2 + (dv + dv_n)^2, above its floor
-        // (the branch taken exactly as the forward takes it)
-        const T du0 = (f0 & F_INU) ? u0 - c.uOc[o] : T(0);
-        const T du1 = (fe & F_INU) ? ue - c.uOc[oe] : T(0);
-        const T dv0 = (f0 & F_INV) ? v0 - c.vOc[o] : T(0);
-        const T dv1 = (fn & F_INV) ? vn - c.vOc[on] : T(0);
-        const T A = du0 + du1, B = dv0 + dv1;
-        const T X = fma(B, B, A * A);
-        const bool south = f0 & F_SOUTH;
-        const bool fast = mC && Fp<T>::gt((south ? k.dcq2S : k.dcq2N) * X, k.cmin2);
         T lX2 = T(0);   // 2 dL/dX
-        if (__any_sync(m, fast)) {
-            const T cd = t.cd[o];
-            const T rc = Fp<T>::rcp(fast ? cd : T(1), m);
-            if (fast) {
-                lX2 = lcd * (south ? k.kXS : k.kXN) * rc;
-                if constexpr (sizeof(T) == 8) a.dragC[o] = fma(lcd, cd, a.dragC[o]);   // reduced once, after the sweep
-                else if (south) dragS = lcd * cd;
-                else dragN = lcd * cd;
-            }
+        if (!EARLY) drag();
+        if (fast) {
+            lX2 = lcd * (south ? k.kXS : k.kXN) * rc;
+            if constexpr (sizeof(T) == 8) a.dragC[o] = fma(lcd, cd, a.dragC[o]);   // reduced once, after the sweep
+            else if (south) dragS = lcd * cd;
+            else dragN = lcd * cd;
         }
         s.ldu[o] = A * lX2;
         s.ldv[o] = B * lX2;
         if (BASAL) {
-            // cb = bfac / sqrt(0.25 (a^2 + b^2 + c^2 + e^2) + U0^2), a = inU u, b = inU_e u_e, c = inV v, e = inV_n v_n
+            if (!EARLY) basal();
             const T lcb = (s.bU[o] + s.bU[oe]) + (s.bV[o] + s.bV[on]);
-            const T a_ = sel<T>(f0 & F_INU, u0), b_ = sel<T>(fe & F_INU, ue);
-            const T c_ = sel<T>(f0 & F_INV, v0), e_ = sel<T>(fn & F_INV, vn);
-            const T qb = T(0.25) * (a_ * a_ + b_ * b_ + c_ * c_ + e_ * e_) + k.U02;
-            const T rs = Fp<T>::rsqrt(qb, m);
             const T bf = c.bfac[o];
             a.bfac[o] += lcb * rs;
             s.lsb[o] = T(-0.25) * bf * rs * rs * rs * lcb;
@@ -615,13 +736,13 @@ __global__ void __launch_bounds__(BX * BY) c_reverse_kernel(Dims d, int64_t lp, 
     c_reverse_body<T, BASAL, TURN>(d, lp, c, t, l, a, k, s);
 }
 
-// On a float32 grid of more CTAs than the GPU holds at once, eight CTAs per
-// SM (32 registers, 20-24 bytes spilled): the latency-bound pass gains more
+// On a float32 grid of more CTAs than the GPU holds at once, 64 warps per
+// SM (32 registers, 32-36 bytes spilled): the latency-bound pass gains more
 // from the resident warps than it loses to the spills (a 0.1-degree reverse
 // step 383.7 -> 375.1 ms); on a grid the GPU holds at once the spills would
 // only cost.
 template <class T, bool BASAL, bool TURN>
-__global__ void __launch_bounds__(BX * BY, 8) c_reverse_occ_kernel(Dims d, int64_t lp, FastConsts<T> c, TapeG<T> t,
+__global__ void __launch_bounds__(BX * BY, 16) c_reverse_occ_kernel(Dims d, int64_t lp, FastConsts<T> c, TapeG<T> t,
                                                                    LamG<T> l, Adj<T> a, KT<T> k, Scr<T> s) {
     c_reverse_body<T, BASAL, TURN>(d, lp, c, t, l, a, k, s);
 }
@@ -720,6 +841,8 @@ __global__ void __launch_bounds__(BX * BY) uv_gather_kernel(Dims d, int64_t lp, 
     const int j = blockIdx.x * BX + threadIdx.x, i = blockIdx.y * BY + threadIdx.y;
     const bool act = i < d.NX && j < d.NY;
     const unsigned m = __ballot_sync(ALL, act);
+    chain_wait();
+    if (k.early) chain_release();
     if (!act) return;
     T lu, lv, luo, lvo;
     p4_point<T, BASAL, TURN>(d, lp, c, t, k, s, m, i, j, lu, lv, luo, lvo);
@@ -745,6 +868,10 @@ __device__ __forceinline__ void uv_link_body(const Dims &d, int64_t lp, const Ha
     const int j = blockIdx.x * BX + threadIdx.x, i = blockIdx.y * BY + threadIdx.y;
     const bool act = i < d.NX && j < d.NY;
     const unsigned m = __ballot_sync(ALL, act);
+    P1Pre<T> q1;
+    if (sizeof(T) == 8 && act) q1 = p1_prepare<T, BASAL>(d, lp, c, t1, k, s, m, i, j);
+    chain_wait();
+    if (k.early) chain_release();
     if (!act) return;
     T lu, lv, luo, lvo;
     p4_point<T, BASAL, false>(d, lp, c, t4, k, s, m, i, j, lu, lv, luo, lvo);
@@ -778,23 +905,25 @@ __device__ __forceinline__ void uv_link_body(const Dims &d, int64_t lp, const Ha
             }
         }
     }
-    p1_point<T, BASAL, false, true>(d, lp, c, t1, l1, a, k, s, m, i, j, LU, LV, luo, lvo);
+    if (sizeof(T) == 4) q1 = p1_prepare<T, BASAL>(d, lp, c, t1, k, s, m, i, j);
+    p1_point<T, BASAL, false, true>(d, lp, c, t1, l1, a, k, s, q1, i, j, LU, LV, luo, lvo);
 }
 
 template <class T, bool BASAL>
-__global__ void __launch_bounds__(BX * BY) uv_link_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<T> c,
+__global__ void __launch_bounds__(BX * BY, sizeof(T) == 8 ? 6 : 1) uv_link_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<T> c,
                                                            TapeG<T> t4, TapeG<T> t1, LamG<T> l4, LamG<T> l1,
                                                            Adj<T> a, KT<T> k, Scr<T> s) {
     uv_link_body<T, BASAL>(d, lp, h, c, t4, t1, l4, l1, a, k, s);
 }
 
-// On a grid of more CTAs than the GPU holds at once, eight CTAs per SM (32
+// On a grid of more CTAs than the GPU holds at once, 64 warps per SM (32
 // registers, spilling).  On 3600 x 1800 a reverse step took 400.0 ms with
-// the passes separate, 428.6 / 401.2 / 389.5 ms with the fused one at four
-// / five / six CTAs per SM, and with P3 at eight CTAs 375.1 ms at six,
-// 364.7 ms at eight.
+// the passes separate, 428.6 / 401.2 / 389.5 ms with the fused one at 32
+// / 40 / 48 warps per SM, and with P3 at 64 warps 375.1 ms at 48, 364.7 ms
+// at 64.  (In float64 the fused pass is bounded to 24 warps: 80 registers
+// and 56 bytes spilled instead of 100 registers, 1440 x 720 5657 -> 5296 us.)
 template <class T, bool BASAL>
-__global__ void __launch_bounds__(BX * BY, 8) uv_link_occ_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<T> c,
+__global__ void __launch_bounds__(BX * BY, 16) uv_link_occ_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<T> c,
                                                                  TapeG<T> t4, TapeG<T> t1, LamG<T> l4, LamG<T> l1,
                                                                  Adj<T> a, KT<T> k, Scr<T> s) {
     uv_link_body<T, BASAL>(d, lp, h, c, t4, t1, l4, l1, a, k, s);
@@ -802,7 +931,7 @@ __global__ void __launch_bounds__(BX * BY, 8) uv_link_occ_kernel(Dims d, int64_t
 
 }  // namespace
 
-// padded cells from which the float32 passes P3 and P4+P1 run at eight CTAs
+// padded cells from which the float32 passes P3 and P4+P1 run at 64 warps
 // per SM (the *_occ_kernel forms; 2^19: 3600 x 1800 faster so; 360 x 180,
 // whose passes fit the GPU at once, slower: 1-degree trajectory 3.75x
 // against 3.53-3.60x)
@@ -842,26 +971,43 @@ static int run_phases(const Dims &d, int64_t lp, const HaloFill &h, const FastCo
         pre_p1<T, B>(d, lp, c, k, t, s, grd, blk, st);
         uv_reverse_kernel<T, B, R><<<grd, blk, 0, st>>>(d, lp, h, c, tt, l, a, k, s);
     }
-    z_reverse_kernel<T><<<grd, blk, 0, st>>>(d, lp, c, tt, l, k, s, t.del == nullptr);
+    int stt = launch_status();
+    if (stt != VERIS_OK) return stt;
+    stt = launch_chained(z_reverse_kernel<T>, grd, blk, 0, st, d, lp, c, tt, l, k, s, t.del == nullptr);
+    if (stt != VERIS_OK) return stt;
     // float32 on a grid of more CTAs than the GPU holds: P3 and the fused pass at eight CTAs per SM
     const bool occupy = sizeof(T) == 4 && (int64_t)d.NX * d.NY >= OCCUPY_CELLS;
-    if constexpr (sizeof(T) == 4) {
-        if (occupy) c_reverse_occ_kernel<T, B, R><<<grd, blk, 0, st>>>(d, lp, c, tt, l, a, k, s);
-        else c_reverse_kernel<T, B, R><<<grd, blk, 0, st>>>(d, lp, c, tt, l, a, k, s);
-    } else {
-        c_reverse_kernel<T, B, R><<<grd, blk, 0, st>>>(d, lp, c, tt, l, a, k, s);
-    }
-    if (tp) {
-        if constexpr (!R && sizeof(T) == 4) {
-            pre_p1<T, B>(d, lp, c, k, *tp, s, grd, blk, st);
-            const TapeG<T> t1 = with_terms(*tp, s);
-            if (occupy) uv_link_occ_kernel<T, B><<<grd, blk, 0, st>>>(d, lp, h, c, tt, t1, l, *lpv, a, k, s);
-            else uv_link_kernel<T, B><<<grd, blk, 0, st>>>(d, lp, h, c, tt, t1, l, *lpv, a, k, s);
-        }
-    } else {
-        uv_gather_kernel<T, B, R><<<grd, blk, 0, st>>>(d, lp, c, tt, l, a, k, s);
+    auto p3 = c_reverse_kernel<T, B, R>;
+    if constexpr (sizeof(T) == 4)
+        if (occupy) p3 = c_reverse_occ_kernel<T, B, R>;
+    if ((stt = launch_chained(p3, grd, blk, 0, st, d, lp, c, tt, l, a, k, s)) != VERIS_OK) return stt;
+    if (!tp) return launch_chained(uv_gather_kernel<T, B, R>, grd, blk, 0, st, d, lp, c, tt, l, a, k, s);
+    if constexpr (!R) {
+        const TapeG<T> t1 = with_terms(*tp, s);
+        auto link = uv_link_kernel<T, B>;
+        if constexpr (sizeof(T) == 4)
+            if (occupy) link = uv_link_occ_kernel<T, B>;
+        if (!B && tp->del)
+            return launch_chained(link, grd, blk, 0, st, d, lp, h, c, tt, t1, l, *lpv, a, k, s);
+        pre_p1<T, B>(d, lp, c, k, *tp, s, grd, blk, st);
+        link<<<grd, blk, 0, st>>>(d, lp, h, c, tt, t1, l, *lpv, a, k, s);
     }
     return launch_status();
+}
+
+// Whether a pass lets its successor's CTAs in as soon as it may write
+// itself, not when it ends.  float64: where the SMs hold two passes at once
+// (up to three CTAs per SM of the six of the fused pass) the successor's
+// part before the wait overlaps the pass: 30-60 subcycles on 90 x 40
+// 1724 -> 1577 us, 180 x 90 1336 -> 1247, 300 x 150 1369 -> 1290, and on
+// grids of several waves it fills the last one: 600 x 300 2340 -> 2225,
+// 1440 x 720 5302 -> 5243.  Between, its CTAs go where the pass left slots
+// and the SMs' shares become uneven: 360 x 180 1580 -> 1707, 443 x 221
+// 1538 -> 1556.  float32, whose passes have nothing before the wait: 360 x 180 926 -> 979.
+template <class T>
+static bool release_early(const Dims &d) {
+    const int64_t ctas = (int64_t)((d.NY + BX - 1) / BX) * ((d.NX + BY - 1) / BY), sms = sm_count();
+    return sizeof(T) == 8 && (ctas <= 3 * sms || ctas > 6 * sms);
 }
 
 template <class T>
@@ -871,7 +1017,8 @@ static int phases(const Dims &d, int64_t lp, const HaloFill &h, const FastConsts
     if (tp && turn) return VERIS_ERR_ARG;   // the link keeps no turning-angle shares
     Scr<T> s;
     std::memcpy(&s, scratch, sizeof s);
-    const KT<T> kk = kt<T>(k, rhoSea);
+    KT<T> kk = kt<T>(k, rhoSea);
+    kk.early = release_early<T>(d);
     if (basal)
         return turn ? run_phases<T, true, true>(d, lp, h, c, kk, t, l, a, s, head, tp, lpv, st)
                     : run_phases<T, true, false>(d, lp, h, c, kk, t, l, a, s, head, tp, lpv, st);
@@ -945,6 +1092,10 @@ template int adjoint_gather_subcycle<float>(const Dims &, int64_t, const HaloFil
                                             const FastScalars<float> &, double, const TapeG<float> &,
                                             const LamG<float> &, const Adj<float> &, float *const[N_SCRATCH], bool,
                                             bool, cudaStream_t);
+template int adjoint_gather_chain<double>(const Dims &, int64_t, const HaloFill &, const FastConsts<double> &,
+                                          const FastScalars<double> &, double, const TapeG<double> &,
+                                          const LamG<double> &, const Adj<double> &, double *const[N_SCRATCH], bool,
+                                          bool, const TapeG<double> *, const LamG<double> *, cudaStream_t);
 template int adjoint_gather_chain<float>(const Dims &, int64_t, const HaloFill &, const FastConsts<float> &,
                                          const FastScalars<float> &, double, const TapeG<float> &,
                                          const LamG<float> &, const Adj<float> &, float *const[N_SCRATCH], bool,
