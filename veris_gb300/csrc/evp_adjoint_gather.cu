@@ -33,9 +33,9 @@
 // before it waits: no pass of the sweep writes those, and what wrote them is
 // complete, since P1 at the head of a sweep and every pass after an
 // unchained kernel start ordinarily.  The wait then covers only the gathers.
-// The sweep on 360 x 180 with its forward, 30 subcycles float64: 1866 us with
-// four passes started one after another, 1580 so; 90 x 40, 60 subcycles 1980
-// and 1577.
+// The sweep on 360 x 180 with its forward, 30 subcycles float64: 1844 us with
+// four passes started one after another, 1576 so; 90 x 40, 60 subcycles 2311
+// and 1591.
 //
 // Every point is computed once, nothing is recomputed on rings and nothing
 // is accumulated with atomics (each input adjoint is written by the pass

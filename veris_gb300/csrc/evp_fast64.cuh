@@ -94,6 +94,15 @@ inline F64Scalars f64_scalars(const FastScalars<double> &k, double sideU0 = 0.0)
 
 // ------------------------------------------------------------------ tile
 constexpr int F64_THREADS = 256, F64_WIDE = 768;
+// Pieces of up to 8 rows in a CTA of 768 threads give its 24 warps fewer tasks
+// than they could take (a 2-row piece has 5 for its viscosities, 2 for its
+// velocities), and a scheduler's float64 pipe serves one warp instruction in 64
+// cycles: two warps of 45 such instructions on one scheduler are the whole
+// stage.  There the drag and Coriolis terms, and U and V points, are tasks of
+// their own.  Per subcycle 90 x 40 8.5 -> 6.6 us, 180 x 90 9.0 -> 7.7,
+// 240 x 121 10.7 -> 9.8; of 9 to 11 rows the warps are busy without and the
+// index work is paid twice: 300 x 150 13.0 -> 13.9, 360 x 180 15.7 -> 16.7.
+constexpr int F64_SPLIT_ROWS = 8;
 
 // TI output rows x 32 columns per CTA; 16-, 24- and 32-row tiles fit 4, 3
 // and 2 CTAs per SM (smaller tiles: more resident warps, more ring work)
@@ -160,13 +169,14 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
     w.unit(blockIdx.x, d.NX, i0, ti, j0);
     // the unit's region sizes (ti <= TI rows)
     const int nS = (ti + 4) * S::WS, nZ = (ti + 3) * S::WZ, nB = (ti + 2) * S::WB, nC = (ti + 1) * S::WC;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
     constexpr unsigned ALL = 0xffffffffu;
 #define IS(li, lj) (((li) + 2) * S::WS + ((lj) + 2))
 #define IZ(li, lj) (((li) + 1) * S::WZ + ((lj) + 1))
 #define IB(li, lj) (((li) + 1) * S::WB + ((lj) + 1))
 #define IC(li, lj) (((li) + 1) * S::WC + ((lj) + 1))
 #define IZZ(li, lj) ((li) * S::WC + (lj))
+    const bool split = NT == F64_WIDE && ti <= F64_SPLIT_ROWS;
     // ocean velocities at tile offsets (read through L1; not staged)
     auto uoc = [&](int li, int lj) { return __ldg(c.uOc + (int64_t)d.wxt(i0 + li) * lp + d.wyt(j0 + lj)); };
     auto voc = [&](int li, int lj) { return __ldg(c.vOc + (int64_t)d.wxt(i0 + li) * lp + d.wyt(j0 + lj)); };
@@ -221,8 +231,57 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
 
     // ---- B: viscosities at C [-1, TI] x [-1, TJ] (veris/dynamics_routines.py:220-268);
     //      stresses, drag and Coriolis terms on [-1, TI) x [-1, TJ) (veris/evp_solver.py:80-145)
-    for (int base = 0; base < nB; base += NT) {
+    auto drag_terms = [&](unsigned m2, int li, int lj, int gi, int gj, int64_t o, uint32_t f0, double u0, double ue,
+                          double v0, double vn, bool own) {
+        const int q = IC(li, lj);
+        const bool mC = f0 & F_MC;
+        // ocean drag at C (veris/dynamics_routines.py:21-52): with X = 4 t and
+        // Y = (dc^2/4) X, dc^2 t > cmin^2 <=> Y > cmin^2 and dc sqrt(t) = sqrt(Y)
+        const uint32_t fe = sF[IS(li + 1, lj)], fn = sF[IS(li, lj + 1)];
+        const double du0 = (f0 & F_INU) ? u0 - __ldg(c.uOc + o) : 0.0;
+        const double du1 = (fe & F_INU) ? ue - uoc(li + 1, lj) : 0.0;
+        const double dv0 = (f0 & F_INV) ? v0 - __ldg(c.vOc + o) : 0.0;
+        const double dv1 = (fn & F_INV) ? vn - voc(li, lj + 1) : 0.0;
+        const double a = du0 + du1, b = dv0 + dv1;
+        const double X = fma(b, b, a * a);
+        const bool south = f0 & F_SOUTH;
+        const double Y = (south ? k.dcq2S : k.dcq2N) * X;
+        const bool fast = gt_nonneg(Y, k.cmin2);
+        double cd = k.cmin;
+        if (__any_sync(m2, fast)) {
+            const double sy = sqrt64(Y, m2);
+            if (fast) cd = sy;
+        }
+        sCd[q] = mC ? cd : 0.0;
+        if (TAPE && own) io.tCd[(int64_t)gi * io.ldo + gj] = mC ? cd : 0.0;
+        if (BASAL) {   // veris/dynamics_routines.py:55-96 with the step factor folded by the prep
+            const double a_ = (f0 & F_INU) ? u0 : 0.0, b_ = (fe & F_INU) ? ue : 0.0;
+            const double c_ = (f0 & F_INV) ? v0 : 0.0, e_ = (fn & F_INV) ? vn : 0.0;
+            const double s = 0.25 * (a_ * a_ + b_ * b_ + c_ * c_ + e_ * e_);
+            sCb[q] = div64(__ldg(c.bfac + o), sqrt64(s + k.U02, m2), m2);
+        }
+        const double mf = __ldg(c.mf4 + o);
+        sFv[q] = mf * (v0 + vn);
+        sFu[q] = mf * (u0 + ue);
+        if (SLIP) {   // veris/dynamics_routines.py:110-112
+            const double us = u0 + ue, vs = v0 + vn;
+            sSp[q] = 0.5 * sqrt64(fma(us, us, vs * vs), m2);
+        }
+    };
+    const int firstD = (nB + 31) / 32 * 32;   // the first drag task's threads
+    for (int base = 0; base < (split ? firstD + nC : nB); base += NT) {
         const int idx = base + tid;
+        if (NT == F64_WIDE && split && idx >= firstD) {   // the drag and Coriolis terms of 32 points
+            const int q = idx - firstD;
+            const unsigned m2 = __ballot_sync(ALL, q < nC);
+            if (q >= nC) continue;
+            const int li = q / S::WC - 1, lj = q % S::WC - 1;
+            const int gi = d.wxt(i0 + li), gj = d.wyt(j0 + lj);
+            drag_terms(m2, li, lj, gi, gj, (int64_t)gi * lp + gj, sF[IS(li, lj)], sU[IS(li, lj)],
+                       sU[IS(li + 1, lj)], sV[IS(li, lj)], sV[IS(li, lj + 1)],
+                       li >= 0 && lj >= 0 && i0 + li < d.NX && j0 + lj < d.NY);
+            continue;
+        }
         const unsigned m = __ballot_sync(ALL, idx < nB);
         if (idx >= nB) continue;
         const int li = idx / S::WB - 1, lj = idx % S::WB - 1;
@@ -276,44 +335,12 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
                 io.s1o[w] = s1;
                 io.s2o[w] = s2;
                 if (AUTO && ADAPT && io.aCo) io.aCo[w] = aC;
+                if (TAPE) {
+                    io.tDel[w] = delta;
+                    io.tZeta[w] = zeta * k.twoAlpha;
+                }
             }
-            // ocean drag at C (veris/dynamics_routines.py:21-52): with X = 4 t and
-            // Y = (dc^2/4) X, dc^2 t > cmin^2 <=> Y > cmin^2 and dc sqrt(t) = sqrt(Y)
-            const uint32_t fe = sF[IS(li + 1, lj)], fn = sF[IS(li, lj + 1)];
-            const double du0 = (f0 & F_INU) ? u0 - __ldg(c.uOc + o) : 0.0;
-            const double du1 = (fe & F_INU) ? ue - uoc(li + 1, lj) : 0.0;
-            const double dv0 = (f0 & F_INV) ? v0 - __ldg(c.vOc + o) : 0.0;
-            const double dv1 = (fn & F_INV) ? vn - voc(li, lj + 1) : 0.0;
-            const double a = du0 + du1, b = dv0 + dv1;
-            const double X = fma(b, b, a * a);
-            const bool south = f0 & F_SOUTH;
-            const double Y = (south ? k.dcq2S : k.dcq2N) * X;
-            const bool fast = gt_nonneg(Y, k.cmin2);
-            double cd = k.cmin;
-            if (__any_sync(m2, fast)) {
-                const double sy = sqrt64(Y, m2);
-                if (fast) cd = sy;
-            }
-            sCd[q] = mC ? cd : 0.0;
-            if (TAPE && own) {
-                const int64_t w = (int64_t)gi * io.ldo + gj;
-                io.tDel[w] = delta;
-                io.tZeta[w] = zeta * k.twoAlpha;
-                io.tCd[w] = mC ? cd : 0.0;
-            }
-            if (BASAL) {   // veris/dynamics_routines.py:55-96 with the step factor folded by the prep
-                const double a_ = (f0 & F_INU) ? u0 : 0.0, b_ = (fe & F_INU) ? ue : 0.0;
-                const double c_ = (f0 & F_INV) ? v0 : 0.0, e_ = (fn & F_INV) ? vn : 0.0;
-                const double s = 0.25 * (a_ * a_ + b_ * b_ + c_ * c_ + e_ * e_);
-                sCb[q] = div64(__ldg(c.bfac + o), sqrt64(s + k.U02, m2), m2);
-            }
-            const double mf = __ldg(c.mf4 + o);
-            sFv[q] = mf * (v0 + vn);
-            sFu[q] = mf * (u0 + ue);
-            if (SLIP) {   // veris/dynamics_routines.py:110-112
-                const double us = u0 + ue, vs = v0 + vn;
-                sSp[q] = 0.5 * sqrt64(fma(us, us, vs * vs), m2);
-            }
+            if (!split) drag_terms(m2, li, lj, gi, gj, o, f0, u0, ue, v0, vn, own);
         }
     }
     __syncthreads();
@@ -348,18 +375,18 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
     chain_release();
 
     // ---- D: u, v at the tile's U and V points (veris/evp_solver.py:105-187)
-    for (int base = 0; base < ti * S::TJ; base += NT) {
-        const int idx = base + tid;
-        const int li = idx / S::TJ, lj = idx % S::TJ;
+    for (int t = tid >> 5; t < (split ? 2 * ti : ti); t += NT / 32) {   // a row's U and V points, or one of the two
+        const bool doU = t < ti, doV = !split || !doU;
+        const int li = doU ? t : t - ti, lj = lane;
         const int gi = i0 + li, gj = j0 + lj;
-        const bool act = idx < ti * S::TJ && gi < d.NX && gj < d.NY;
+        const bool act = gi < d.NX && gj < d.NY;
         const unsigned m = __ballot_sync(ALL, act);
         if (!act) continue;
         const int64_t o = (int64_t)gi * lp + gj;
         const uint32_t f0 = sF[IS(li, lj)];
         const double u0 = sU[IS(li, lj)], v0 = sV[IS(li, lj)];
         const double cd0 = sCd[IC(li, lj)], cdw = sCd[IC(li - 1, lj)], cds = sCd[IC(li, lj - 1)];
-        {   // U point
+        if (doU) {   // U point
             const double kU = __ldg(c.hAW + o) * (cd0 + cdw);
             const double uo0 = __ldg(c.uOc + o);
             double fx = fma(kU, uo0, __ldg(c.cU + o)) + (sFv[IC(li, lj)] + sFv[IC(li - 1, lj)]);
@@ -398,7 +425,7 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
             }
             store_filled_ld(io.uo, io.ldo, d, h, gi, gj, un);
         }
-        {   // V point
+        if (doV) {   // V point
             const double kV = __ldg(c.hAS + o) * (cd0 + cds);
             const double vo0 = __ldg(c.vOc + o);
             double fy = fma(kV, vo0, __ldg(c.cV + o)) - (sFu[IC(li, lj)] + sFu[IC(li, lj - 1)]);
@@ -464,9 +491,9 @@ static int launch64_tile(const Dims &d, int64_t lp, const HaloFill &h, const Fas
 
 // Grids that one 16-row piece per SM covers take one CTA of 768 threads per SM:
 // as many warps as three of 256, on pieces three times as tall, whose rings are
-// a smaller part of the work.  Per subcycle, three CTAs / one: 128 x 64
-// 10.4 / 8.6 us, 180 x 90 11.0 / 9.0, 240 x 121 12.3 / 10.7, 360 x 180 17.1 / 15.8;
-// with taller pieces the three win, 443 x 221 23.5 / 25.0, 600 x 300 35.0 / 45.6.
+// a smaller part of the work.  Per subcycle, three CTAs / one (without split
+// tasks): 128 x 64 10.4 / 8.6 us, 180 x 90 11.0 / 9.0, 240 x 121 12.3 / 10.7,
+// 360 x 180 17.1 / 15.8; with taller pieces the three win, 443 x 221 23.5 / 25.0, 600 x 300 35.0 / 45.6.
 // (384 threads x 2: 9.5, 9.5, 11.5, 16.9; 512 x 1: 8.4, 8.7, 10.5, 18.9.)
 template <int TI, bool B, bool R, bool TP, bool AD = false, bool SL = false, bool AUTO = false>
 static int launch64(const Dims &d, int64_t lp, const HaloFill &h, const FastConsts<double> &c, const F64Scalars &k,
