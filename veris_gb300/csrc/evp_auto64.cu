@@ -13,7 +13,8 @@
 // curvature terms, finite inputs) is only known on the device, so the once-per-
 // call preparation, which reads every field anyway, leaves the answer in a
 // word that the subcycle kernel branches on: no synchronisation, the same
-// launches either way, usable under stream capture.
+// launches either way, usable under stream capture.  On small grids an eager
+// call runs the whole loop in one launch.
 //
 // The folded constants and half of the ping-pong state take the caller's
 // pitch, so that everything the subcycle reads unchanged (ocean velocities,
@@ -22,6 +23,8 @@
 #include "evp_residual.cuh"
 
 namespace veris {
+
+constexpr size_t AUTO_STATUS_BYTES = 256;   // the state check's word, and at +128 the loop's barrier count
 
 struct AutoSpace {
     int *viol;
@@ -39,7 +42,7 @@ static size_t auto_layout(const Dims &d, const VerisParams &p, char *base, AutoS
     auto take = [&](size_t n) { char *q = base ? base + off : nullptr; off += n; return q; };
     auto field = [&](bool used) { return used ? reinterpret_cast<double *>(take(f2)) : nullptr; };
     const bool adapt = p.useAdaptiveEVP != 0, slip = p.noSlip == 0, basal = p.basalDragK2 != 0.0;
-    a->viol = reinterpret_cast<int *>(take(256));
+    a->viol = reinterpret_cast<int *>(take(AUTO_STATUS_BYTES));
     a->ctx = reinterpret_cast<Ctx<double> *>(take(rup256(sizeof(Ctx<double>))));
     FastConsts<double> &c = a->c;
     c = FastConsts<double>{};
@@ -195,6 +198,17 @@ static int auto_launch(bool adapt, bool slip, const Dims &d, const HaloFill &h, 
                 : launch64<24, B, R, false, false, false, true>(d, d.ld, h, c, k, io, st, a);
 }
 
+// the whole loop in one launch, on the grids that take it
+template <bool B, bool R>
+static int auto_loop_launch(bool adapt, bool slip, const Dims &d, const HaloFill &h, const FastConsts<double> &c,
+                            const F64Scalars &k, const F64Loop &l, cudaStream_t st, const F64Auto &a) {
+    if (adapt)
+        return slip ? launch64_loop<B, R, true, true>(d, d.ld, h, c, k, l, st, a)
+                    : launch64_loop<B, R, true, false>(d, d.ld, h, c, k, l, st, a);
+    return slip ? launch64_loop<B, R, false, true>(d, d.ld, h, c, k, l, st, a)
+                : launch64_loop<B, R, false, false>(d, d.ld, h, c, k, l, st, a);
+}
+
 // where a loop with residual diagnostics keeps alphaC and the partial sums
 struct AutoResidual {
     double *aC, *partial;
@@ -204,7 +218,7 @@ struct AutoResidual {
 // sums after each
 static int auto_loop(const Dims &d, const VerisParams *p, const VerisFieldsF64 *vs, AutoSpace &a, int n, double *u,
                      double *v, double *s1, double *s2, double *s12, const AutoResidual *res, cudaStream_t st) {
-    if (cudaMemsetAsync(a.viol, 0, sizeof(int), st) != cudaSuccess) return VERIS_ERR_LAUNCH;
+    if (cudaMemsetAsync(a.viol, 0, AUTO_STATUS_BYTES, st) != cudaSuccess) return VERIS_ERR_LAUNCH;
     Ctx<double> x;
     x.f = *reinterpret_cast<const Fields<double> *>(vs);
     x.d = d;
@@ -230,6 +244,27 @@ static int auto_loop(const Dims &d, const VerisParams *p, const VerisFieldsF64 *
                turn = p->sinWat != 0.0;
     double *const outs[5] = {u, v, s1, s2, s12};
     const double *cur[5] = {x.f.uIce, x.f.vIce, x.f.sigma1, x.f.sigma2, x.f.sigma12};
+    // a graph has no host time per launch to save
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const bool eager = cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+    if (!eager) cudaGetLastError();
+    if (!res && eager) {
+        F64Loop l;
+        for (int q = 0; q < 5; ++q) {
+            l.in[q] = cur[q];
+            l.even[q] = (n - 1) % 2 ? a.state[q] : outs[q];
+            l.odd[q] = (n - 1) % 2 ? outs[q] : a.state[q];
+            l.out[q] = outs[q];
+        }
+        l.ldo = d.ld;
+        l.n = n;
+        l.arrived = reinterpret_cast<unsigned *>(a.viol) + 32;
+        stt = basal ? (turn ? auto_loop_launch<true, true>(adapt, slip, d, h, c, k, l, st, aa)
+                            : auto_loop_launch<true, false>(adapt, slip, d, h, c, k, l, st, aa))
+                    : (turn ? auto_loop_launch<false, true>(adapt, slip, d, h, c, k, l, st, aa)
+                            : auto_loop_launch<false, false>(adapt, slip, d, h, c, k, l, st, aa));
+        if (stt == VERIS_OK) return stt;   // else one launch per subcycle
+    }
     for (int it = 0; it < n; ++it) {
         double *const *dst = (n - 1 - it) % 2 ? a.state : outs;
         FastIO<double> io{cur[0], cur[1], cur[2], cur[3], cur[4], dst[0], dst[1], dst[2], dst[3], dst[4], d.ld};

@@ -94,6 +94,18 @@ inline F64Scalars f64_scalars(const FastScalars<double> &k, double sideU0 = 0.0)
 
 // ------------------------------------------------------------------ tile
 constexpr int F64_THREADS = 256, F64_WIDE = 768;
+constexpr int F64_LOOP_ROWS = 16;
+
+// a loop of n subcycles: the first reads `in`, subcycle it < n - 1 writes
+// `even` or `odd` (pitch of the inputs), the last `out` (pitch ldo)
+struct F64Loop {
+    const double *in[5];
+    double *even[5], *odd[5], *out[5];
+    int64_t ldo;
+    int n;
+    unsigned *arrived;   // zero at the launch
+};
+
 // Pieces of up to 8 rows in a CTA of 768 threads give its 24 warps fewer tasks
 // than they could take (a 2-row piece has 5 for its viscosities, 2 for its
 // velocities), and a scheduler's float64 pipe serves one warp instruction in 64
@@ -144,10 +156,12 @@ __device__ __noinline__ void plain_fallback(const Ctx<double> *ctx, HaloFill h, 
     plain_tile<double, TI, ADAPT, SLIP, BASAL, NT>(smem_raw, *c, h, p, i0, ti, j0);
 }
 
-template <int TI, bool BASAL, bool TURN, bool TAPE, bool ADAPT, bool SLIP, bool AUTO, int NT>
-__global__ void __launch_bounds__(NT, NT > F64_THREADS ? 1 : ((ADAPT || SLIP) ? 3 : f64_min_blocks(TI)))
-evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars k, FastIO<double> io,
-               TileUnits w, F64Auto a) {
+// rows [i0, i0 + ti) and the 32 columns from j0 of one subcycle.  LOOP: one of
+// a launch that runs the whole loop (no successor to start)
+template <int TI, bool BASAL, bool TURN, bool TAPE, bool ADAPT, bool SLIP, bool AUTO, int NT, bool LOOP>
+__device__ __forceinline__ void f64_tile(const Dims &d, int64_t lp, const HaloFill &h, const FastConsts<double> &c,
+                                         const F64Scalars &k, const FastIO<double> &io, const F64Auto &a, int i0,
+                                         int ti, int j0) {
     using S = Smem64<TI>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *sU = reinterpret_cast<double *>(smem_raw);
@@ -165,8 +179,6 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
     double *sA = sSp + (SLIP ? S::NC : 0);     // adaptive alpha only
     uint32_t *sF = reinterpret_cast<uint32_t *>(sA + (ADAPT ? S::NB : 0));
     double *sS12 = sZq;
-    int i0, ti, j0;
-    w.unit(blockIdx.x, d.NX, i0, ti, j0);
     // the unit's region sizes (ti <= TI rows)
     const int nS = (ti + 4) * S::WS, nZ = (ti + 3) * S::WZ, nB = (ti + 2) * S::WB, nC = (ti + 1) * S::WC;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -181,13 +193,6 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
     auto uoc = [&](int li, int lj) { return __ldg(c.uOc + (int64_t)d.wxt(i0 + li) * lp + d.wyt(j0 + lj)); };
     auto voc = [&](int li, int lj) { return __ldg(c.vOc + (int64_t)d.wxt(i0 + li) * lp + d.wyt(j0 + lj)); };
 
-    chain_wait();
-    if (AUTO) {
-        if (*a.viol) {   // the same for every CTA and subcycle
-            plain_fallback<TI, ADAPT, SLIP, BASAL, NT>(a.ctx, h, io, i0, ti, j0);
-            return;
-        }
-    }
     // ---- stage u, v and the flags of the tile plus a 2-cell ring
     for (int idx = tid; idx < nS; idx += NT) {
         const int li = idx / S::WS - 2, lj = idx % S::WS - 2;
@@ -372,7 +377,7 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
     // 191.0 us a subcycle on 1440 x 720, before C 191.4, before B 191.1, at
     // the kernel's start 192.1, unchained 194.0; 360 x 180: 20.1, 20.5, 20.8,
     // 21.2, 22.6)
-    chain_release();
+    if (!LOOP) chain_release();
 
     // ---- D: u, v at the tile's U and V points (veris/evp_solver.py:105-187)
     for (int t = tid >> 5; t < (split ? 2 * ti : ti); t += NT / 32) {   // a row's U and V points, or one of the two
@@ -472,6 +477,78 @@ evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars 
 #undef IZZ
 }
 
+template <int TI, bool BASAL, bool TURN, bool TAPE, bool ADAPT, bool SLIP, bool AUTO, int NT>
+__global__ void __launch_bounds__(NT, NT > F64_THREADS ? 1 : ((ADAPT || SLIP) ? 3 : f64_min_blocks(TI)))
+evp_f64_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars k, FastIO<double> io,
+               TileUnits w, F64Auto a) {
+    int i0, ti, j0;
+    w.unit(blockIdx.x, d.NX, i0, ti, j0);
+    chain_wait();
+    if (AUTO) {
+        if (*a.viol) {   // the same for every CTA and subcycle
+            plain_fallback<TI, ADAPT, SLIP, BASAL, NT>(a.ctx, h, io, i0, ti, j0);
+            return;
+        }
+    }
+    f64_tile<TI, BASAL, TURN, TAPE, ADAPT, SLIP, AUTO, NT, false>(d, lp, h, c, k, io, a, i0, ti, j0);
+}
+
+// the n subcycles of a unit, `tile` one of them; false if a barrier gave up
+template <class F>
+__device__ __forceinline__ bool f64_loop(const F64Loop &l, int64_t lp, F tile) {
+    FastIO<double> io{l.in[0], l.in[1], l.in[2], l.in[3], l.in[4]};
+    for (int it = 0;; ++it) {
+        const bool last = it == l.n - 1;
+        double *const *to = last ? l.out : (it & 1 ? l.odd : l.even);
+        io.uo = to[0];
+        io.vo = to[1];
+        io.s1o = to[2];
+        io.s2o = to[3];
+        io.s12o = to[4];
+        io.ldo = last ? l.ldo : lp;
+        tile(io);
+        if (last) return true;
+        if (!grid_barrier(l.arrived, it + 1)) return false;
+        io.u = io.uo;
+        io.v = io.vo;
+        io.s1 = io.s1o;
+        io.s2 = io.s2o;
+        io.s12 = io.s12o;
+    }
+}
+
+// A whole loop of n subcycles in one launch, one unit per CTA.  The barrier
+// between two subcycles takes what starting the next of a chain of launches
+// takes or a little more (a subcycle on 90 x 40 6.7 us chained, 6.7 so,
+// 180 x 90 7.8 and 8.0, 240 x 121 10.0 and 10.0, 360 x 180 15.5 and 15.7).
+// What goes is the host's 5.5 us per launch, which a chain of short subcycles
+// does not cover once the host has more to do: a step on 90 x 40 with 120 of
+// them takes 1066 us instead of 1393.
+template <bool BASAL, bool TURN, bool ADAPT, bool SLIP>
+__global__ void __launch_bounds__(F64_WIDE, 1)
+evp_f64_loop_kernel(Dims d, int64_t lp, HaloFill h, FastConsts<double> c, F64Scalars k, F64Loop l, TileUnits w,
+                    F64Auto a) {
+    constexpr int TI = F64_LOOP_ROWS, NT = F64_WIDE;
+    int i0, ti, j0;
+    w.unit(blockIdx.x, d.NX, i0, ti, j0);
+    bool done;
+    if (*a.viol)
+        done = f64_loop(l, lp, [&](const FastIO<double> &io) {
+            plain_fallback<TI, ADAPT, SLIP, BASAL, NT>(a.ctx, h, io, i0, ti, j0);
+        });
+    else
+        done = f64_loop(l, lp, [&](const FastIO<double> &io) {
+            f64_tile<TI, BASAL, TURN, false, ADAPT, SLIP, true, NT, true>(d, lp, h, c, k, io, a, i0, ti, j0);
+        });
+    if (done) return;
+    for (int q = threadIdx.x; q < ti * 32; q += NT) {   // given up: no number stands for a result
+        const int gi = i0 + q / 32, gj = j0 + q % 32;
+        if (gi < d.NX && gj < d.NY)
+            for (int f = 0; f < 5; ++f)
+                l.out[f][(int64_t)gi * l.ldo + gj] = __longlong_as_double(0x7ff8000000000000ll);
+    }
+}
+
 template <int TI, bool B, bool R, bool TP, bool AD, bool SL, bool AUTO, int NT>
 static int launch64_tile(const Dims &d, int64_t lp, const HaloFill &h, const FastConsts<double> &c, const F64Scalars &k,
                     const FastIO<double> &io, cudaStream_t st, const F64Auto &a) {
@@ -498,9 +575,30 @@ static int launch64_tile(const Dims &d, int64_t lp, const HaloFill &h, const Fas
 template <int TI, bool B, bool R, bool TP, bool AD = false, bool SL = false, bool AUTO = false>
 static int launch64(const Dims &d, int64_t lp, const HaloFill &h, const FastConsts<double> &c, const F64Scalars &k,
                     const FastIO<double> &io, cudaStream_t st, const F64Auto &a = F64Auto{}) {
-    const int stt = launch64_tile<16, B, R, TP, AD, SL, AUTO, F64_WIDE>(d, lp, h, c, k, io, st, a);
+    const int stt = launch64_tile<F64_LOOP_ROWS, B, R, TP, AD, SL, AUTO, F64_WIDE>(d, lp, h, c, k, io, st, a);
     if (stt != VERIS_ERR_UNSUPPORTED) return stt;
     return launch64_tile<TI, B, R, TP, AD, SL, AUTO, F64_THREADS>(d, lp, h, c, k, io, st, a);
+}
+
+// The drop-in's loop in one launch, where the pieces are short enough that the
+// host's time per launch shows (evp_f64_loop_kernel); VERIS_ERR_UNSUPPORTED,
+// having launched nothing, on larger grids.
+template <bool B, bool R, bool AD, bool SL>
+static int launch64_loop(const Dims &d, int64_t lp, const HaloFill &h, const FastConsts<double> &c,
+                         const F64Scalars &k, const F64Loop &l, cudaStream_t st, const F64Auto &a) {
+    using S = Smem64<F64_LOOP_ROWS>;
+    auto kern = evp_f64_loop_kernel<B, R, AD, SL>;
+    const size_t sm = S::bytes(B, AD, SL);
+    static std::atomic<bool> configured[MAX_DEVICES];
+    if (!smem_configured(configured, kern, (int)sm)) return VERIS_ERR_LAUNCH;
+    static std::atomic<int> resident[MAX_DEVICES];
+    const int slots = cta_slots(resident, kern, F64_WIDE, sm);
+    if (slots <= 0) return VERIS_ERR_LAUNCH;
+    if ((int64_t)((d.NY + S::TJ - 1) / S::TJ) * ((d.NX + F64_LOOP_ROWS - 1) / F64_LOOP_ROWS) > slots)
+        return VERIS_ERR_UNSUPPORTED;
+    const TileUnits w = tile_units(d, F64_LOOP_ROWS, slots);
+    if ((d.NX + w.P1 - 1) / w.P1 > F64_SPLIT_ROWS) return VERIS_ERR_UNSUPPORTED;
+    return launch_cooperative(kern, dim3(w.count), dim3(F64_WIDE), sm, st, d, lp, h, c, k, l, w, a);
 }
 
 }  // namespace veris
