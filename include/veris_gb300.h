@@ -679,10 +679,8 @@ int veris_convert_f64_to_f32(const double *src, float *dst, int64_t n, veris_str
 int veris_convert_f32_to_f64(const float *src, double *dst, int64_t n, veris_stream_t s);
 /*
  * No counterpart in the reference: a self-check of the float64 division,
- * reciprocal and square roots that the float64 kernels take from the
- * hardware's approximate reciprocal and reciprocal square root refined by
- * the series of the exact correction (instead of IEEE division and square
- * root).  For n operand pairs (a, b) in device memory it writes 8 planar
+ * reciprocal and square roots that the float64 kernels evaluate in integer
+ * and float32 instructions (instead of IEEE division and square root).  For n operand pairs (a, b) in device memory it writes 8 planar
  * arrays of n values to out: a/b, a/b, 1/b, 1/b, sqrt(b), sqrt(b),
  * 1/sqrt(b), 1/sqrt(b), each pair in the warp-uniform form (a warp with any
  * operand outside the safe range takes IEEE for all its lanes) and in the
@@ -692,8 +690,9 @@ int veris_convert_f32_to_f64(const float *src, double *dst, int64_t n, veris_str
  * (sqrt of -0 in the warp form: +0 when the warp takes the series).
  */
 int veris_f64_math_check(const double *a, const double *b, int64_t n, double *out, veris_stream_t s);
-/* The float64 kernels' table-driven exp(x), log(x) and atan(x), planar in out
- * (3 n values), for checking them against correctly rounded results. */
+/* The float64 kernels' table-driven exp(x) and the bulk formula's psi_m and
+ * psi_h at s = x, planar in out (3 n values), for checking them against
+ * correctly rounded results. */
 int veris_f64_functions_check(const double *x, int64_t n, double *out, veris_stream_t s);
 
 #ifdef __cplusplus

@@ -1,7 +1,7 @@
 // Float64 arithmetic off the float64 pipe, for kernels that it bounds: GB300
 // has 2 float64 lanes per SM and cycle, 1/64 of its float32 rate.  Division and
 // square root in integer and float32 instructions, comparisons and conversions
-// on the integer pipe, table-driven exponential, logarithm and arctangent; the
+// on the integer pipe, a table-driven exponential and psi functions; the
 // reciprocal square root from the hardware's seed and the series of the exact
 // correction.  No slow paths inside: a lane or warp whose operands leave a safe
 // exponent range takes IEEE division or square root instead.
@@ -263,35 +263,40 @@ __device__ __forceinline__ double exp_table(double x) {
     return (unsigned)(__double2hiint(x) & 0x7fffffff) < 0x4085e000u ? exp_core(x) : exp_far(x);
 }
 
-// log(x) for x = 2^e m in [1, 2^64): with r = m c - 1, c ~ 1/m from the table,
-// log x = e ln2 - log c + r + r^2 (-1/2 + r (1/3 + r (-1/4 + r/5))).  Other x: log().
-__device__ __forceinline__ double log_table(double x) {
-    const int hi = __double2hiint(x);
-    if ((unsigned)(hi - 0x3ff00000) >= (64u << 20)) return ::log(x);
-    const double m = __hiloint2double((hi & 0x000fffff) | 0x3ff00000, __double2loint(x));
-    const double2 c = __ldg(LOG_256 + ((hi >> 12) & 255));
-    const double r = fma(m, c.x, -1.0);
-    const float f = narrow(r);
-    const double t = widen(f * fmaf(f, fmaf(f, -1.f / 6.f, 0.2f), -0.25f));
-    const double p = fma(r * r, fma(r, 1.0 / 3.0 + t, -0.5), r);
-    const int e = (hi - 0x3ff00000) >> 20;
-    double L = c.y;
-    if (e != 0) L = fma(widen((float)e), 0.6931471805599453094, L);
-    return L + p;
-}
-
-// atan(x) for x in [1, 3.6]: with c the nearest 1 + k/64 and d = (x - c)/(1 + x c),
-// atan x = atan c + d + d^3 (-1/3 + d^2 (1/5 - d^2/7)).  Other x: atan().
-__device__ __forceinline__ double atan_table(double x) {
-    const int hi = __double2hiint(x);
-    if ((unsigned)(hi - 0x3ff00000) > (unsigned)(0x400ccccc - 0x3ff00000)) return ::atan(x);
-    const int k = (int)fmaf(narrow(x), 64.f, -63.5f);   // 64 (x - 1), rounded
-    const double c = widen(fmaf((float)k, 0.015625f, 1.f));
-    const double d = div_int(x - c, fma(x, c, 1.0));
-    const double d2 = d * d;
-    const float f = narrow(d2);
-    const double q = widen(f * fmaf(f, -1.f / 7.f, 0.2f)) - 1.0 / 3.0;
-    return __ldg(ATAN_64 + k) + fma(d * d2, q, d);
-}
+// The bulk formula's psi_m and psi_h at s = 1 - 16 huol in [1, 161]
+//   psi_m = 2 ln((1 + x)/2) + 2 ln((1 + x^2)/2) - 2 atan x + pi/2,
+//   psi_h = 2 ln((1 + x^2)/2), x = s^(1/4)
+// from their series about the nearest of 32 points an octave (|t| <= 2^-6: the
+// float32 part, from t^5 on, is below 2^-34 of 1), 12 float64 operations for
+// both.  Absolute error at most 9e-16 and 5e-16 (4000 points against 200-bit
+// values; with the float64 square roots, logarithms and arctangent 1.5e-15).
+// The tables are read by random index: in shared memory, one plane per coefficient.
+struct PsiTables {
+    double head[10 * PSI_POINTS];
+    float tail[8 * PSI_POINTS], r[32];
+    __device__ __forceinline__ void load(int threads) {
+        for (int q = threadIdx.x; q < 10 * PSI_POINTS; q += threads) head[q] = PSI_HEAD[q];
+        for (int q = threadIdx.x; q < 8 * PSI_POINTS; q += threads) tail[q] = PSI_TAIL[q];
+        if (threadIdx.x < 32) r[threadIdx.x] = PSI_R[threadIdx.x];
+    }
+    // a NaN's or larger s takes the last point: NaN, or no value of use
+    __device__ __forceinline__ void eval(double s, double &psim, double &psih) const {
+        const unsigned at = (unsigned)(__double2hiint(s) - 0x3ff00000) >> 15;
+        const int n = at < PSI_POINTS ? (int)at : PSI_POINTS - 1;
+        const double c = widen(r[n & 31]);
+        const double t = fma(s, __hiloint2double(__double2hiint(c) - ((n >> 5) << 20), __double2loint(c)), -1.0);
+        const float f = narrow(t);
+        auto series = [&](const double *h, const float *l) {
+            const float e = f * fmaf(f, fmaf(f, fmaf(f, l[3 * PSI_POINTS], l[2 * PSI_POINTS]), l[PSI_POINTS]), l[0]);
+            double p = h[4 * PSI_POINTS] + widen(e);
+            p = fma(p, t, h[3 * PSI_POINTS]);
+            p = fma(p, t, h[2 * PSI_POINTS]);
+            p = fma(p, t, h[PSI_POINTS]);
+            return fma(p, t, h[0]);
+        };
+        psim = series(head + n, tail + n);
+        psih = series(head + 5 * PSI_POINTS + n, tail + 4 * PSI_POINTS + n);
+    }
+};
 
 }  // namespace veris

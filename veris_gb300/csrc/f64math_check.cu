@@ -3,7 +3,7 @@
 // bulk formula use them in place of IEEE division and square root): each
 // form evaluated elementwise, so that a caller can measure them against
 // correctly rounded results and IEEE special values; and of its table-driven
-// exponential, logarithm and arctangent (Growth, the bulk formula).
+// exponential (Growth, the bulk formula) and the bulk formula's psi functions.
 #include "common.cuh"
 #include "f64math.cuh"
 
@@ -33,13 +33,15 @@ __global__ void __launch_bounds__(CHECK_THREADS) f64math_check_kernel(const doub
     out[7 * n + i] = rsqrt_lane(y);
 }
 
-// out (planar, n each): exp_table(x), log_table(x), atan_table(x)
+// out (planar, n each): exp_table(x), psi_m and psi_h (s = x)
 __global__ void __launch_bounds__(CHECK_THREADS) f64functions_check_kernel(const double *x, int64_t n, double *out) {
+    __shared__ PsiTables psi;
+    psi.load(CHECK_THREADS);
+    __syncthreads();
     const int64_t i = (int64_t)blockIdx.x * CHECK_THREADS + threadIdx.x;
     if (i >= n) return;
     out[i] = exp_table(x[i]);
-    out[n + i] = log_table(x[i]);
-    out[2 * n + i] = atan_table(x[i]);
+    psi.eval(x[i], out[n + i], out[2 * n + i]);
 }
 
 }  // namespace

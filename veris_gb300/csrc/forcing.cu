@@ -235,18 +235,24 @@ __global__ void __launch_bounds__(256) bulkf_kernel(BulkArgs<T> a) {
 }
 
 // The float64 bulk formula, bound by the float64 pipe: the scheme of
-// bulkf_kernel with the table-driven logarithm, arctangent and exponential
-// (7, 11 and 8 float64 operations), square roots and reciprocals without
-// range checks where the scheme bounds the operand, comparisons on the
-// integer pipe, and the iteration's constants folded: 32 float64 operations
-// per unstable iteration, two per stable one.
-//   psi_m = 2 ln((1 + x)/2) + 2 ln((1 + x^2)/2) - 2 atan x + pi/2,
-//   psi_h = 2 ln((1 + x^2)/2), x = (1 - 16 huol)^(1/4);
+// bulkf_kernel with psi_m and psi_h from one table of their series in
+// s = 1 - 16 huol (12 float64 operations instead of two square roots, two
+// logarithms and an arctangent), a table-driven exponential, square roots and
+// reciprocals without range checks where the scheme bounds the operand,
+// comparisons on the integer pipe, and the iteration's constants folded: 17
+// float64 operations per unstable iteration, two per stable one.
 //   Dm, Dh = 1 + g (aln - psi) = c0 - g psi
 // 1444 x 724 points, half of them unstable: 1.50 ms with CUDA's log, atan and
-// exp (170 operations per unstable iteration); 0.67 ms with reciprocal and
-// square root series on the float64 pipe; here 0.48 ms.
-__global__ void __launch_bounds__(256) bulkf64_kernel(BulkArgs<double> a, double c0) {
+// exp (170 operations per unstable iteration); 0.48 ms with table-driven ones,
+// 32 operations; here 0.30 ms, 725 x 363 121 -> 82 us with the call.  Eight
+// CTAs per SM, each with the tables in its shared memory: six 309 and 92 us,
+// four 305 and 92, three 292 and 91.
+constexpr int BULK64_BLOCKS = 8;
+
+__global__ void __launch_bounds__(256, BULK64_BLOCKS) bulkf64_kernel(BulkArgs<double> a, double c0) {
+    __shared__ PsiTables psi;
+    psi.load(256);
+    __syncthreads();
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < a.n;
          k += (int64_t)gridDim.x * blockDim.x) {
         const double uw = __ldg(a.uw + k), vw = __ldg(a.vw + k);
@@ -266,14 +272,10 @@ __global__ void __launch_bounds__(256) bulkf64_kernel(BulkArgs<double> a, double
             if ((unsigned)(__double2hiint(h) & 0x7fffffff) >= 0x40240000u && !is_nan64(h))
                 h = __hiloint2double((__double2hiint(h) & 0x80000000) | 0x40240000, 0);
             if (is_neg(h)) {
-                const double s = sqrt_int(fma(-16.0, h, 1.0));
-                const double xsq = __double2hiint(s) < 0x3ff00000 ? 1.0 : s;
-                const double x = sqrt_int(xsq);
-                const double l2 = 2.0 * log_table(fma(0.5, xsq, 0.5));
-                const double lx = log_table(fma(0.5, x, 0.5));
-                const double psim = fma(-2.0, atan_table(x), fma(2.0, lx, l2)) + 1.57079632679489661923;
+                double psim, psih;
+                psi.eval(fma(-16.0, h, 1.0), psim, psih);
                 Dm = fma(-a.g, psim, c0);
-                Dh = fma(-a.g, l2, c0);
+                Dh = fma(-a.g, psih, c0);
                 if (it == 4) break;
                 h = div_lane(K * (Dm * Dm), Dh);
             } else {   // stable (or neutral, or NaN): both psi are -5 huol, the unstable terms carry a factor 0
@@ -362,7 +364,7 @@ static int bulkf(const VerisParams *p, int64_t n, const T *uw, const T *vw, cons
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t want = (n + 255) / 256;
-    const int64_t cap = (int64_t)(sms > 0 ? sms : 148) * 8;
+    const int64_t cap = (int64_t)(sms > 0 ? sms : 148) * (sizeof(T) == 8 ? BULK64_BLOCKS : 8);
     const int blocks = (int)(want < cap ? want : cap);
     if constexpr (sizeof(T) == 8) bulkf64_kernel<<<blocks, 256, 0, (cudaStream_t)s>>>(a, 1.0 + a.g * a.aln);
     else bulkf_kernel<T><<<blocks, 256, 0, (cudaStream_t)s>>>(a);
