@@ -10,8 +10,8 @@
 // masks of 1 are not multiplied, the transport, Courant number and update
 // factor serve all fields, a slope is formed once, and warps without ice (four
 // zero values around the face in every field) skip the flux.
-// 1444 x 724, three fields: 549 us in five launches; here 79 and 76 us (float64
-// pipe 74 and 76 % busy).
+// 1444 x 724, three fields: 549 us in five launches; here 68 and 71 us (float64
+// pipe 68 and 73 % busy; 79 and 76 us with the divisions on it).
 //
 // Face i of axis 0 (j of axis 1) takes field values f[i-2 .. i+1]; the fluxes
 // vanish outside [2, N-2] and the halo fill that the reference applies to them

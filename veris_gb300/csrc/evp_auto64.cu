@@ -4,10 +4,10 @@
 // The plain loop (evp.cu) evaluates every option with the reference's order of
 // operations and IEEE division: 210 float64 operations per cell and subcycle
 // and more against the folded form's 90, on a GPU whose float64 pipe is what
-// binds.  A call of 12 subcycles, per subcycle, plain (32-row tiles) / folded:
-//   90 x 40      104 / 16 us     with adaptive, side, basal and turned terms 183 / 16
-//   360 x 180    104 / 22                                                   185 / 40
-//   1440 x 720   690 / 206                                                 1092 / 433
+// binds.  Per subcycle, plain (32-row tiles) / folded:
+//   90 x 40      104 / 6.7 us    with adaptive, side, basal and turned terms 183 / 9.0
+//   360 x 180    104 / 15.6                                                  185 / 26.6
+//   1440 x 720   690 / 167                                                 1092 / 320
 // and 19, 60, 657 us (30, 96, 1022) on states left to the plain tile.  Whether a state is one the
 // folded form covers (metrics that vary along one axis, masks 0 or 1, no
 // curvature terms, finite inputs) is only known on the device, so the once-per-

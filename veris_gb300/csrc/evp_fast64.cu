@@ -23,9 +23,9 @@ static int launch64_rows(const Dims &d, int64_t lp, const HaloFill &h, const Fas
 
 // rows per tile of later float64 subcycles (0: the default); process-wide
 static std::atomic<int> g_tile_rows{0};
-// measured on GB300 (ordered units): 24 rows 204.0 / 1153.0 us per subcycle
-// on 1440x720 / 3600x1800, against 202.6 / 1173.3 (16) and 222.7 / 1240.8
-// (32); the bench's tuner picks per workload
+// 24 rows 171.5 us per subcycle on 1440x720 (unchained, cold start), 16 rows
+// 172.5, 32 rows 202.1; 3600x1800 927 us (24) and 933 (16); the bench's tuner
+// picks per workload
 constexpr int F64_DEFAULT_ROWS = 24;
 
 int fast64_subcycle(const Dims &d, const HaloFill &h, const FastConsts<double> &c, const FastScalars<double> &ks,
