@@ -608,6 +608,7 @@ struct Plan {
     T *cp, *seg, *lam[2][5];
     T *scr[N_SCRATCH];   // the gather passes' arrays
     size_t field;   // bytes of one internal array
+    size_t zero;    // bytes from the first constant adjoint to be cleared
     size_t total;
 };
 
@@ -619,12 +620,14 @@ static size_t plan(const Dims &d, int n, int K, char *base, Plan<T> *pl, bool ta
     auto take = [&](size_t nb) { char *q = base ? base + off : nullptr; off += nb; return q; };
     T **arrs[11] = {&pl->a.Ph, &pl->a.mfC, &pl->a.bfac, &pl->a.mU, &pl->a.cU, &pl->a.AW, &pl->a.uOc,
                     &pl->a.mV, &pl->a.cV, &pl->a.AS, &pl->a.vOc};
+    const size_t first = off;
     for (int q = 0; q < 11; ++q) *arrs[q] = reinterpret_cast<T *>(take(pl->field));
     double *sc = reinterpret_cast<double *>(take(256));
     pl->a.dragN = sc;
     pl->a.dragS = sc ? sc + 1 : nullptr;
     // float64 gather passes: per-cell water-drag sums, reduced after the sweep
     pl->a.dragC = reinterpret_cast<double *>(take(sizeof(T) == 8 ? rup256((size_t)d.NX * lp * sizeof(double)) : 0));
+    pl->zero = off - first;
     const int ncp = taped ? 0 : (n + K - 1) / K;
     pl->cp = reinterpret_cast<T *>(take((size_t)ncp * 5 * pl->field));
     pl->seg = reinterpret_cast<T *>(take(taped ? 0 : (size_t)(K + 1) * 5 * pl->field));
@@ -693,15 +696,9 @@ static int evp_adjoint(const VerisGrid *g, const VerisParams *p, const VerisFiel
     const HaloFill h = halo_fill_of(*p);
     const FastScalars<T> k = fast_scalars<T>(*p);
     int stt;
-    // zero the constant adjoints and the scalars
-    T *zero_list[11] = {pl.a.Ph, pl.a.mfC, pl.a.bfac, pl.a.mU, pl.a.cU, pl.a.AW, pl.a.uOc,
-                        pl.a.mV, pl.a.cV, pl.a.AS, pl.a.vOc};
-    for (int q = 0; q < 11; ++q)
-        if (cudaMemsetAsync(zero_list[q], 0, pl.field, st) != cudaSuccess) return VERIS_ERR_LAUNCH;
-    if (cudaMemsetAsync(pl.a.dragN, 0, 2 * sizeof(double), st) != cudaSuccess) return VERIS_ERR_LAUNCH;
-    if (sizeof(T) == 8 &&
-        cudaMemsetAsync(pl.a.dragC, 0, (size_t)d.NX * lp * sizeof(double), st) != cudaSuccess)
-        return VERIS_ERR_LAUNCH;
+    // the constant adjoints, the scalars and (float64) the per-cell drag sums, which lie
+    // together, in one call instead of thirteen (360 x 180, 30 subcycles: 1566 -> 1527 us)
+    if (cudaMemsetAsync(pl.a.Ph, 0, pl.zero, st) != cudaSuccess) return VERIS_ERR_LAUNCH;
 
     // forward sweep: state 0 from the prep, checkpoints every K subcycles
     T *cp0[5];

@@ -570,7 +570,8 @@ static int launch64_tile(const Dims &d, int64_t lp, const HaloFill &h, const Fas
 // as many warps as three of 256, on pieces three times as tall, whose rings are
 // a smaller part of the work.  Per subcycle, three CTAs / one (without split
 // tasks): 128 x 64 10.4 / 8.6 us, 180 x 90 11.0 / 9.0, 240 x 121 12.3 / 10.7,
-// 360 x 180 17.1 / 15.8; with taller pieces the three win, 443 x 221 23.5 / 25.0, 600 x 300 35.0 / 45.6.
+// 360 x 180 17.1 / 15.8; with taller pieces the three win, 443 x 221 23.5 / 25.0,
+// 600 x 300 35.0 / 45.6.
 // (384 threads x 2: 9.5, 9.5, 11.5, 16.9; 512 x 1: 8.4, 8.7, 10.5, 18.9.)
 template <int TI, bool B, bool R, bool TP, bool AD = false, bool SL = false, bool AUTO = false>
 static int launch64(const Dims &d, int64_t lp, const HaloFill &h, const FastConsts<double> &c, const F64Scalars &k,
